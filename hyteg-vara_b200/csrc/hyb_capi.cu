@@ -364,10 +364,10 @@ int hyb_function_interpolate_const( hyb_function* fh, int level, double value, i
    if ( value == 0.0 && flag == HYB_ALL )
       HYB_CUDA( cudaMemsetAsync( f->at( level ), 0, f->levelBytes( level ), S( stream ) ) );
    else if ( f->dtype == HYB_F64 )
-      k_fill< double ><<< dim3( L.slabBlocks, f->st->td.nC ), 256, 0, S( stream ) >>>( f->st->td, L.dev,
+      k_fill< double ><<< dim3( L.vecBlocks, f->st->td.nC ), kVecThreads, 0, S( stream ) >>>( f->st->td, L.dev,
                                                                                       f->ptr< double >( level ), value, flag );
    else
-      k_fill< float ><<< dim3( L.slabBlocks, f->st->td.nC ), 256, 0, S( stream ) >>>( f->st->td, L.dev,
+      k_fill< float ><<< dim3( L.vecBlocks, f->st->td.nC ), kVecThreads, 0, S( stream ) >>>( f->st->td, L.dev,
                                                                                      f->ptr< float >( level ), float( value ),
                                                                                      flag );
    HYB_CHECK_LAUNCH();
@@ -1075,13 +1075,13 @@ int hyb_function_dot_noalloc( hyb_function* ah, hyb_function* bh, int level, int
    double* scratch = noAllocScratch();
    // every slot the reduction reads is rewritten by the first pass, so nothing is cleared
    if ( a->dtype == HYB_F64 )
-      k_dot_partial< double ><<< dim3( L.slabBlocks, st.td.nC ), 256, 0, S( stream ) >>>(
+      k_dot_partial< double ><<< dim3( L.vecBlocks, st.td.nC ), kVecThreads, 0, S( stream ) >>>(
           st.td, L.dev, a->ptr< double >( level ), b->ptr< double >( level ), flag, scratch, nullptr );
    else
-      k_dot_partial< float ><<< dim3( L.slabBlocks, st.td.nC ), 256, 0, S( stream ) >>>(
+      k_dot_partial< float ><<< dim3( L.vecBlocks, st.td.nC ), kVecThreads, 0, S( stream ) >>>(
           st.td, L.dev, a->ptr< float >( level ), b->ptr< float >( level ), flag, scratch, nullptr );
    HYB_CHECK_LAUNCH();
-   k_reduce_final<<< 1, 1024, 0, S( stream ) >>>( scratch, int( slots ), out_device );
+   k_reduce_final<<< 1, 1024, 0, S( stream ) >>>( scratch, L.vecBlocks * st.td.nC, out_device );
    HYB_CHECK_LAUNCH();
    HYB_API_END
 }

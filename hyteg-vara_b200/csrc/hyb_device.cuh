@@ -21,6 +21,14 @@
 
 namespace hyb {
 
+// Programmatic dependent launch: a kernel lets the next kernel of its stream be scheduled
+// as soon as all its blocks run (launch_dependents), and every kernel waits for the
+// previous one to complete and its memory to be visible before touching any data (wait).
+// Launches with cudaLaunchAttributeProgrammaticStreamSerialization thus overlap the launch
+// latency of a kernel with the tail of its predecessor; without the attribute both
+// instructions do nothing.
+#define HYB_PDL_PROLOGUE() asm volatile( "griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory" )
+
 struct ClassDev
 {
    int32_t id;    // primitive id within its kind
@@ -57,6 +65,7 @@ struct LevelDev
    int     nSeg;               // interior row segments (32 points each)
    const int32_t* seg;         // packed z | y<<10 | x0<<20
    const int32_t* xyz;         // closure index -> x | y<<10 | z<<20
+   const int32_t* linPos;      // slab position of each interior point, in tet-linear order
    // Cell-interior points, the same for every cell of the level. A block is a run of
    // interior points at consecutive storage positions whose 15 neighbours sit at the same
    // offsets (a residue group x = 4g + r of one row, r fixed); blk[16 b + q] is the

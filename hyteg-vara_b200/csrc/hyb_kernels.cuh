@@ -23,13 +23,7 @@ enum ApplyMode : int
                       // accumulate into *acc, and float(r) goes to cvt when given
 };
 
-// Programmatic dependent launch: a kernel lets the next kernel of its stream be scheduled
-// as soon as all its blocks run (launch_dependents), and every kernel waits for the
-// previous one to complete and its memory to be visible before touching any data (wait).
-// Launches with cudaLaunchAttributeProgrammaticStreamSerialization thus overlap the launch
-// latency of a kernel with the tail of its predecessor; without the attribute both
-// instructions do nothing.
-#define HYB_PDL_PROLOGUE() asm volatile( "griddepcontrol.launch_dependents;\n\tgriddepcontrol.wait;" ::: "memory" )
+constexpr int kAllFlags = 15; // every DoFType bit a DoF can have (HYB_ALL)
 
 constexpr int kCellWarps  = 4; // warps (row segments) per cell block
 constexpr int kBdryThreads = 128;
@@ -2316,30 +2310,126 @@ __global__ void __launch_bounds__( 128 ) k_restrict( TopoDev tp, LevelDev lv, in
 
 // ---------------------------------------------------------------------------
 // Pointwise vector kernels over whole cell slabs (all replicas; consistent by
-// construction). blockIdx.y = cell.
+// construction). blockIdx.y = cell. They are DRAM bound once a thread has several 16-byte
+// loads in flight and the per-point work is small: a thread takes kVecWidth consecutive
+// values (slabs start on 256-byte boundaries), and the boundary flags of the cell's 16
+// point classes are read once per block into a 16-bit mask instead of once per point. One
+// value per thread with a class-table read per point took 125 us for a two-term FP64
+// combination of 18.4 M slab values (3.5 TB/s) and 103 us for a dot product (2.9 TB/s), and
+the dot's 72 k partial sums another 35 us in the reduction's one block; an FP64 copy of 17.6 M
+values went from 85 to 42 us (6.7 TB/s).
 // ---------------------------------------------------------------------------
+constexpr int kVecWidth   = 4;
+constexpr int kVecThreads = 256;
+constexpr int kVecBlock   = kVecWidth * kVecThreads; // slab values per block
+
+// bit m set: the points of class mask m of the cell have a boundary flag in `flag` (and,
+// with owned, their canonical replica is in this cell). All threads of the block call it.
+__device__ __forceinline__ unsigned classFlags( const TopoDev& tp, int cell, int flag, bool owned )
+{
+   __shared__ unsigned bits;
+   if ( threadIdx.x < 32 )
+   {
+      bool on = false;
+      if ( threadIdx.x < 16 )
+      {
+         const ClassDev& cd = tp.cls[cell * 16 + int( threadIdx.x )];
+         on                 = ( cd.bc & flag ) && ( !owned || cd.owned );
+      }
+      const unsigned b = __ballot_sync( 0xffffffffu, on );
+      if ( threadIdx.x == 0 )
+         bits = b;
+   }
+   __syncthreads();
+   return bits;
+}
+
+// kVecWidth consecutive values of a slab, moved with 16-byte accesses
 template < typename T >
-__global__ void k_lincomb( TopoDev tp, LevelDev lv, T* __restrict__ dst, int n, T s0, const T* a0, T s1, const T* a1, T s2,
-                           const T* a2, int add, int flag )
+struct alignas( 16 ) Vec
+{
+   T v[kVecWidth];
+};
+
+// the values of the block's thread: first slab position, and bit e set for each of the
+// kVecWidth points whose class is in `classes`
+struct VecPoints
+{
+   int      idx;
+   unsigned on;
+};
+__device__ __forceinline__ VecPoints vecPoints( const LevelDev& lv, unsigned classes )
+{
+   VecPoints P{ int( blockIdx.x * kVecBlock + threadIdx.x * kVecWidth ), 0 };
+   if ( P.idx >= lv.S )
+      return P;
+   if ( classes == 0xffffu )
+      P.on = 0xf;
+   else
+   {
+      if ( P.idx + kVecWidth <= lv.S )
+      {
+         const int4 p    = __ldg( reinterpret_cast< const int4* >( lv.xyz + P.idx ) );
+         const int  q[4] = { p.x, p.y, p.z, p.w };
+#pragma unroll
+         for ( int e = 0; e < kVecWidth; ++e )
+            P.on |= ( ( classes >> classMask( lv.N, q[e] & 1023, ( q[e] >> 10 ) & 1023, q[e] >> 20 ) ) & 1u ) << e;
+      }
+      else
+         for ( int e = 0; P.idx + e < lv.S; ++e )
+         {
+            const int q = lv.xyz[P.idx + e];
+            P.on |= ( ( classes >> classMask( lv.N, q & 1023, ( q >> 10 ) & 1023, q >> 20 ) ) & 1u ) << e;
+         }
+   }
+   if ( P.idx + kVecWidth > lv.S )
+      P.on &= ( 1u << ( lv.S - P.idx ) ) - 1u; // the slab's padding is never written
+   return P;
+}
+// all kVecWidth values in one go, or the flagged ones
+template < typename T >
+__device__ __forceinline__ void vecStore( T* dst, const Vec< T >& r, unsigned on )
+{
+   if ( on == 0xf )
+      *reinterpret_cast< Vec< T >* >( dst ) = r;
+   else
+#pragma unroll
+      for ( int e = 0; e < kVecWidth; ++e )
+         if ( on & ( 1u << e ) )
+            dst[e] = r.v[e];
+}
+
+// dst may be one of the sources: a thread reads its values of every operand before it writes
+template < typename T >
+__global__ void __launch_bounds__( kVecThreads ) k_lincomb( TopoDev tp, LevelDev lv, T* dst, int n, T s0, const T* a0,
+                                                            T s1, const T* a1, T s2, const T* a2, int add, int flag )
 {
    HYB_PDL_PROLOGUE();
-   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-   if ( idx >= lv.S )
+   const int       cell = blockIdx.y;
+   const VecPoints P    = vecPoints( lv, flag == kAllFlags ? 0xffffu : classFlags( tp, cell, flag, false ) );
+   if ( !P.on )
       return;
-   const int cell = blockIdx.y;
-   const int p    = lv.xyz[idx];
-   const int mask = classMask( lv.N, p & 1023, ( p >> 10 ) & 1023, p >> 20 );
-   if ( !( tp.cls[cell * 16 + mask].bc & flag ) )
-      return;
-   const size_t i = size_t( cell ) * lv.stride + idx;
-   T            v = add ? dst[i] : T( 0 );
+   const size_t i = size_t( cell ) * lv.stride + P.idx;
+   Vec< T >     r{}, a, b, c;
+   if ( add )
+      r = *reinterpret_cast< const Vec< T >* >( dst + i );
    if ( n > 0 )
-      v += s0 * a0[i];
+      a = *reinterpret_cast< const Vec< T >* >( a0 + i );
    if ( n > 1 )
-      v += s1 * a1[i];
+      b = *reinterpret_cast< const Vec< T >* >( a1 + i );
    if ( n > 2 )
-      v += s2 * a2[i];
-   dst[i] = v;
+      c = *reinterpret_cast< const Vec< T >* >( a2 + i );
+#pragma unroll
+   for ( int e = 0; e < kVecWidth; ++e )
+   {
+      if ( n > 0 )
+         r.v[e] += s0 * a.v[e];
+      if ( n > 1 )
+         r.v[e] += s1 * b.v[e];
+      if ( n > 2 )
+         r.v[e] += s2 * c.v[e];
+   }
+   vecStore( dst + i, r, P.on );
 }
 
 // ---------------------------------------------------------------------------
@@ -2514,17 +2604,13 @@ __global__ void k_fill_tet_factors( LevelDev lv, const double* __restrict__ cell
 
 // VertexDoFFunction::interpolate(constant, level, flag)
 template < typename T >
-__global__ void k_fill( TopoDev tp, LevelDev lv, T* __restrict__ dst, T value, int flag )
+__global__ void __launch_bounds__( kVecThreads ) k_fill( TopoDev tp, LevelDev lv, T* __restrict__ dst, T value, int flag )
 {
    HYB_PDL_PROLOGUE();
-   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-   if ( idx >= lv.S )
-      return;
-   const int cell = blockIdx.y;
-   const int p    = lv.xyz[idx];
-   const int mask = classMask( lv.N, p & 1023, ( p >> 10 ) & 1023, p >> 20 );
-   if ( tp.cls[cell * 16 + mask].bc & flag )
-      dst[size_t( cell ) * lv.stride + idx] = value;
+   const int       cell = blockIdx.y;
+   const VecPoints P    = vecPoints( lv, classFlags( tp, cell, flag, false ) );
+   if ( P.on )
+      vecStore( dst + size_t( cell ) * lv.stride + P.idx, Vec< T >{ { value, value, value, value } }, P.on );
 }
 
 template < typename TD, typename TS >
@@ -2538,44 +2624,53 @@ __global__ void k_convert( LevelDev lv, TD* __restrict__ dst, const TS* __restri
 
 // x64 += e (FP32 correction) on flagged points
 template < typename T, typename TE >
-__global__ void k_add_correction( TopoDev tp, LevelDev lv, T* __restrict__ x, const TE* __restrict__ e, int flag )
+__global__ void __launch_bounds__( kVecThreads ) k_add_correction( TopoDev tp, LevelDev lv, T* __restrict__ x,
+                                                                   const TE* __restrict__ e, int flag )
 {
    HYB_PDL_PROLOGUE();
-   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-   if ( idx >= lv.S )
+   const int       cell = blockIdx.y;
+   const VecPoints P    = vecPoints( lv, classFlags( tp, cell, flag, false ) );
+   if ( !P.on )
       return;
-   const int cell = blockIdx.y;
-   const int p    = lv.xyz[idx];
-   const int mask = classMask( lv.N, p & 1023, ( p >> 10 ) & 1023, p >> 20 );
-   if ( !( tp.cls[cell * 16 + mask].bc & flag ) )
-      return;
-   const size_t i = size_t( cell ) * lv.stride + idx;
-   x[i] += T( e[i] );
+   const size_t    i = size_t( cell ) * lv.stride + P.idx;
+   Vec< T >        r = *reinterpret_cast< const Vec< T >* >( x + i );
+   const Vec< TE > c = *reinterpret_cast< const Vec< TE >* >( e + i );
+#pragma unroll
+   for ( int k = 0; k < kVecWidth; ++k )
+      r.v[k] += T( c.v[k] );
+   vecStore( x + i, r, P.on );
 }
 
-// Partial dot products over the canonical replica of every DoF whose BC is in flag. With
-// cvt given, the pass also writes float(a) at every closure point (the mixed-precision
-// refinement's FP32 right-hand side from the FP64 residual, read once for both).
+// Partial dot products over the canonical replica of every DoF whose BC is in flag, one per
+// block of kVecBlock slab values. With cvt given, the pass also writes float(a) at every
+// closure point (the mixed-precision refinement's FP32 right-hand side from the FP64
+// residual, read once for both).
 template < typename T >
-__global__ void k_dot_partial( TopoDev tp, LevelDev lv, const T* __restrict__ a, const T* __restrict__ b, int flag,
-                               double* __restrict__ partial, float* __restrict__ cvt )
+__global__ void __launch_bounds__( kVecThreads ) k_dot_partial( TopoDev tp, LevelDev lv, const T* __restrict__ a,
+                                                                const T* __restrict__ b, int flag,
+                                                                double* __restrict__ partial, float* __restrict__ cvt )
 {
    HYB_PDL_PROLOGUE();
    __shared__ double red[32];
-   const int idx  = blockIdx.x * blockDim.x + threadIdx.x;
-   const int cell = blockIdx.y;
-   double    v    = 0;
-   if ( idx < lv.S )
+   const int         cell = blockIdx.y;
+   const VecPoints   P    = vecPoints( lv, classFlags( tp, cell, flag, true ) );
+   const size_t      i    = size_t( cell ) * lv.stride + P.idx;
+   double            v    = 0;
+   if ( P.on || ( cvt && P.idx < lv.S ) )
    {
+      const Vec< T > x = *reinterpret_cast< const Vec< T >* >( a + i );
+      const Vec< T > y = *reinterpret_cast< const Vec< T >* >( b + i );
+#pragma unroll
+      for ( int e = 0; e < kVecWidth; ++e )
+         if ( P.on & ( 1u << e ) )
+            v += double( x.v[e] ) * double( y.v[e] );
       if ( cvt )
-         cvt[size_t( cell ) * lv.stride + idx] = float( a[size_t( cell ) * lv.stride + idx] );
-      const int p    = lv.xyz[idx];
-      const int mask = classMask( lv.N, p & 1023, ( p >> 10 ) & 1023, p >> 20 );
-      const ClassDev cd = tp.cls[cell * 16 + mask];
-      if ( cd.owned && ( cd.bc & flag ) )
       {
-         const size_t i = size_t( cell ) * lv.stride + idx;
-         v              = double( a[i] ) * double( b[i] );
+         Vec< float > f;
+#pragma unroll
+         for ( int e = 0; e < kVecWidth; ++e )
+            f.v[e] = float( x.v[e] );
+         vecStore( cvt + i, f, P.idx + kVecWidth <= lv.S ? 0xfu : ( 1u << ( lv.S - P.idx ) ) - 1u );
       }
    }
    for ( int o = 16; o > 0; o >>= 1 )
@@ -2617,50 +2712,59 @@ __global__ void k_reduce_final( const double* __restrict__ partial, int n, doubl
 }
 
 // Canonical DoF order <-> cell slabs (see oracle/hyteg_oracle.h for the order).
-__device__ __forceinline__ int64_t canonicalDof( const TopoDev& tp, const LevelDev& lv, int cell, int x, int y, int z )
+// The cell interiors of the canonical vector are contiguous per cell, in tet-linear order:
+// LevelDev::linPos gives the slab position of each, so a point costs one table read, one
+// slab access (a warp's accesses fall into the four residue runs of a row or two) and one
+// coalesced canonical access. Blocks [0, nIntBlocks) of a cell's row of blocks take its
+// interior, the blocks behind them, over all cells, the surface DoFs, a thread each. Deriving
+// every point's canonical number from its coordinates (class table, tetrahedral indices) was
+// issue bound: 98 us for 18.4 M slab values in FP64 and 93 us in FP32, now 45 and 34 us.
+template < typename T, bool TO >
+__global__ void __launch_bounds__( kVecThreads ) k_dofs( TopoDev tp, LevelDev lv, int nIntBlocks, T* __restrict__ slab,
+                                                         T* __restrict__ dofs )
 {
-   const int       N    = lv.N;
-   const int       mask = classMask( N, x, y, z );
-   const ClassDev& cd   = tp.cls[cell * 16 + mask];
-   const int       b[4] = { N - x - y - z, x, y, z };
-   const int64_t   offE = tp.nV, offF = offE + int64_t( tp.nE ) * ( N - 1 ), offC = offF + int64_t( tp.nF ) * lv.nIntFace;
-   switch ( cd.kind )
+   HYB_PDL_PROLOGUE();
+   const int cell = blockIdx.y;
+   if ( int( blockIdx.x ) < nIntBlocks )
    {
-   case 0: return cd.id;
-   case 1: return offE + int64_t( cd.id ) * ( N - 1 ) + ( b[cd.k1] - 1 );
-   case 2: {
-      const int i = b[cd.k1], j = b[cd.k2];
-      return offF + int64_t( cd.id ) * lv.nIntFace + ( j - 1 ) * ( N - 1 ) - ( j - 1 ) * j / 2 + ( i - 1 );
+      T* const s = slab + size_t( cell ) * lv.stride;
+      T* const d = dofs + ( tp.nV + int64_t( tp.nE ) * ( lv.N - 1 ) + int64_t( tp.nF ) * lv.nIntFace +
+                            int64_t( cell ) * lv.nIntCell );
+      int      at[kVecWidth];
+      T        v[kVecWidth];
+      const int i0 = int( blockIdx.x ) * kVecBlock + int( threadIdx.x );
+#pragma unroll
+      for ( int e = 0; e < kVecWidth; ++e )
+      {
+         const int i = i0 + e * kVecThreads;
+         at[e]       = i < lv.nIntCell ? __ldg( lv.linPos + i ) : -1;
+      }
+#pragma unroll
+      for ( int e = 0; e < kVecWidth; ++e )
+         if ( at[e] >= 0 )
+            v[e] = TO ? s[at[e]] : d[i0 + e * kVecThreads];
+#pragma unroll
+      for ( int e = 0; e < kVecWidth; ++e )
+         if ( at[e] >= 0 )
+         {
+            if ( TO )
+               d[i0 + e * kVecThreads] = v[e];
+            else
+               s[at[e]] = v[e];
+         }
+      return;
    }
-   default: return offC + int64_t( cell ) * lv.nIntCell + cidx( N - 3, x - 1, y - 1, z - 1 );
+   // surface DoFs are numbered as decodeBdry counts them
+   const int nb = int( gridDim.x ) - nIntBlocks;
+   for ( int t = ( cell * nb + int( blockIdx.x ) - nIntBlocks ) * kVecThreads + int( threadIdx.x ); t < lv.nBdry;
+         t += tp.nC * nb * kVecThreads )
+   {
+      const BdryPoint p = decodeBdry( tp, lv, t );
+      if ( TO )
+         dofs[t] = slab[bdryReplica< T >( tp, lv, p, 0 )];
+      else
+         bdryWriteAll( tp, lv, p, slab, dofs[t] );
    }
-}
-
-template < typename T >
-__global__ void k_from_dofs( TopoDev tp, LevelDev lv, T* __restrict__ slab, const T* __restrict__ dofs )
-{
-   HYB_PDL_PROLOGUE();
-   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-   if ( idx >= lv.S )
-      return;
-   const int cell = blockIdx.y;
-   const int p    = lv.xyz[idx];
-   slab[size_t( cell ) * lv.stride + idx] = dofs[canonicalDof( tp, lv, cell, p & 1023, ( p >> 10 ) & 1023, p >> 20 )];
-}
-
-template < typename T >
-__global__ void k_to_dofs( TopoDev tp, LevelDev lv, const T* __restrict__ slab, T* __restrict__ dofs )
-{
-   HYB_PDL_PROLOGUE();
-   const int idx = blockIdx.x * blockDim.x + threadIdx.x;
-   if ( idx >= lv.S )
-      return;
-   const int cell = blockIdx.y;
-   const int p    = lv.xyz[idx];
-   const int x = p & 1023, y = ( p >> 10 ) & 1023, z = p >> 20;
-   if ( !tp.cls[cell * 16 + classMask( lv.N, x, y, z )].owned )
-      return;
-   dofs[canonicalDof( tp, lv, cell, x, y, z )] = slab[size_t( cell ) * lv.stride + idx];
 }
 
 // ---------------------------------------------------------------------------

@@ -7,20 +7,25 @@
 // ---------------------------------------------------------------------------
 inline int bdryBlocks( const LevelDev& d ) { return ( d.nBdry + kBdryThreads - 1 ) / kBdryThreads; }
 
+// canonical vector -> slabs (TO = false) or slabs -> canonical vector
+template < typename T, bool TO >
+void launchDofs( const Storage& s, int l, T* slab, T* dofs, cudaStream_t stream )
+{
+   const auto& L    = s.L( l );
+   const int   nInt = ( L.dev.nIntCell + kVecBlock - 1 ) / kVecBlock;
+   const int   nSrf = int( ( L.dev.nBdry + long( kVecThreads ) * s.td.nC - 1 ) / ( long( kVecThreads ) * s.td.nC ) );
+   pdlLaunch( k_dofs< T, TO >, dim3( nInt + nSrf, s.td.nC ), dim3( kVecThreads ), 0, stream, s.td, L.dev, nInt, slab, dofs );
+   HYB_CHECK_LAUNCH();
+}
 template < typename T >
 void launchFromDofs( const Storage& s, int l, T* slab, const T* dofs, cudaStream_t stream )
 {
-   const auto& L = s.L( l );
-   pdlLaunch( k_from_dofs< T >, dim3( dim3( L.slabBlocks, s.td.nC ) ), dim3( 256 ), 0, stream, s.td, L.dev, slab, dofs );
-   HYB_CHECK_LAUNCH();
+   launchDofs< T, false >( s, l, slab, const_cast< T* >( dofs ), stream );
 }
-
 template < typename T >
 void launchToDofs( const Storage& s, int l, const T* slab, T* dofs, cudaStream_t stream )
 {
-   const auto& L = s.L( l );
-   pdlLaunch( k_to_dofs< T >, dim3( dim3( L.slabBlocks, s.td.nC ) ), dim3( 256 ), 0, stream, s.td, L.dev, slab, dofs );
-   HYB_CHECK_LAUNCH();
+   launchDofs< T, true >( s, l, const_cast< T* >( slab ), dofs, stream );
 }
 
 // Levels whose closure slabs hold at most this many points (all cells) get full row tables
@@ -725,7 +730,7 @@ void launchLincomb( const Storage& s, int l, T* dst, int n, const double* sc, co
                     cudaStream_t stream )
 {
    const auto& L = s.L( l );
-   pdlLaunch( k_lincomb< T >, dim3( dim3( L.slabBlocks, s.td.nC ) ), dim3( 256 ), 0, stream, s.td, L.dev, dst, n, T( n > 0 ? sc[0] : 0 ), n > 0 ? src[0] : nullptr, T( n > 1 ? sc[1] : 0 ),
+   pdlLaunch( k_lincomb< T >, dim3( L.vecBlocks, s.td.nC ), dim3( kVecThreads ), 0, stream, s.td, L.dev, dst, n, T( n > 0 ? sc[0] : 0 ), n > 0 ? src[0] : nullptr, T( n > 1 ? sc[1] : 0 ),
        n > 1 ? src[1] : nullptr, T( n > 2 ? sc[2] : 0 ), n > 2 ? src[2] : nullptr, add ? 1 : 0, flag );
    HYB_CHECK_LAUNCH();
 }
@@ -737,10 +742,10 @@ void launchDot( const Storage& s, int l, const T* a, const T* b, int flag, doubl
                 cudaStream_t stream, float* cvt = nullptr )
 {
    const auto& L = s.L( l );
-   pdlLaunch( k_dot_partial< T >, dim3( dim3( L.slabBlocks, s.td.nC ) ), dim3( 256 ), 0, stream, s.td, L.dev, a, b, flag, partial,
+   pdlLaunch( k_dot_partial< T >, dim3( L.vecBlocks, s.td.nC ), dim3( kVecThreads ), 0, stream, s.td, L.dev, a, b, flag, partial,
               cvt );
    HYB_CHECK_LAUNCH();
-   pdlLaunch( k_reduce_final, dim3( 1 ), dim3( 1024 ), 0, stream, partial, L.slabBlocks * s.td.nC, result );
+   pdlLaunch( k_reduce_final, dim3( 1 ), dim3( 1024 ), 0, stream, partial, L.vecBlocks * s.td.nC, result );
    HYB_CHECK_LAUNCH();
 }
 
@@ -788,7 +793,7 @@ template < typename T >
 void launchAddCorrection( const Storage& s, int l, double* x, const T* e, int flag, cudaStream_t stream )
 {
    const auto& L = s.L( l );
-   pdlLaunch( k_add_correction< double, T >, dim3( dim3( L.slabBlocks, s.td.nC ) ), dim3( 256 ), 0, stream, s.td, L.dev, x, e, flag );
+   pdlLaunch( k_add_correction< double, T >, dim3( L.vecBlocks, s.td.nC ), dim3( kVecThreads ), 0, stream, s.td, L.dev, x, e, flag );
    HYB_CHECK_LAUNCH();
 }
 

@@ -22,7 +22,7 @@ struct LevelHost
    std::unique_ptr< RowTables > rows; // built on first use (ensureRows)
    bool                         rowsTried = false;
    std::unique_ptr< RowTables > blendRows; // full rows for blending operators (ensureBlendRows)
-   DevBuf< int32_t >  seg, xyz, blk, blkXYZ, pts, ptsC, quads, rowYZ;
+   DevBuf< int32_t >  seg, xyz, linPos, blk, blkXYZ, pts, ptsC, quads, rowYZ;
    DevBuf< int32_t >  lexCell, lexCellOff, lexFace, lexFaceOff; // LevelDev::lex* (ensureLex)
    DevBuf< int4 >     lexCellNbr;                                  // LevelDev::lexCellNbr
    DevBuf< int32_t >  lexOfPts, lexSidx;                           // LevelDev::lexOfPts, lexSidx
@@ -36,6 +36,7 @@ struct LevelHost
    int                colourBlocks = 0;  // grid of the loops over one interior colour
    int                bdryBlocks   = 0;  // grid of the surface-DoF loops
    int                slabBlocks   = 0;  // blocks of 256 over one closure
+   int                vecBlocks    = 0;  // blocks of kVecBlock over one closure
 };
 
 struct Storage
@@ -335,6 +336,14 @@ void buildStorage( Storage& s, const std::vector< std::array< double, 3 > >& V, 
          for ( int y = 0; y <= d.N - z; ++y )
             for ( int x = 0; x <= d.N - y - z; ++x )
                xyz[sidx( d.W, x, y, z )] = x | ( y << 10 ) | ( z << 20 );
+      std::vector< int32_t > linPos;
+      for ( int z = 1; z <= d.N; ++z )
+         for ( int y = 1; y + z <= d.N - 2; ++y )
+            for ( int x = 1; x + y + z <= d.N - 1; ++x )
+               linPos.push_back( sidx( d.W, x, y, z ) );
+      require( int( linPos.size() ) == d.nIntCell, "interior point count" );
+      lh->linPos.upload( linPos );
+      d.linPos = lh->linPos.p;
       lh->seg.upload( seg );
       lh->xyz.upload( xyz );
       d.nSeg = int( seg.size() );
@@ -353,6 +362,7 @@ void buildStorage( Storage& s, const std::vector< std::array< double, 3 > >& V, 
       lh->colourBlocks = grid( long( ( maxColour + 31 ) / 32 ) * nC, kCellWarps, 16 );
       lh->bdryBlocks    = grid( bdryLaneCount( nV, nE * ( d.N - 1 ), nF * d.nIntFace ), kBdryThreads, 8 );
       lh->slabBlocks    = ( d.S + 255 ) / 256;
+      lh->vecBlocks     = ( d.S + kVecBlock - 1 ) / kVecBlock;
       maxPartial        = std::max( maxPartial, size_t( lh->slabBlocks ) * nC );
       // surface DoFs grouped by SOR colour: colour = sum of label(v) * micro-weight(v) over
       // the primitive's vertices (the same value in every adjacent cell)
