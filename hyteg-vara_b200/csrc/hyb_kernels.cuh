@@ -2316,8 +2316,8 @@ __global__ void __launch_bounds__( 128 ) k_restrict( TopoDev tp, LevelDev lv, in
 // point classes are read once per block into a 16-bit mask instead of once per point. One
 // value per thread with a class-table read per point took 125 us for a two-term FP64
 // combination of 18.4 M slab values (3.5 TB/s) and 103 us for a dot product (2.9 TB/s), and
-the dot's 72 k partial sums another 35 us in the reduction's one block; an FP64 copy of 17.6 M
-values went from 85 to 42 us (6.7 TB/s).
+// the dot's 72 k partial sums another 35 us in the reduction's one block; an FP64 copy of
+// 17.6 M values went from 85 to 42 us (6.7 TB/s).
 // ---------------------------------------------------------------------------
 constexpr int kVecWidth   = 4;
 constexpr int kVecThreads = 256;
