@@ -344,11 +344,95 @@ struct OpDev
    int            bN;     // micro-edges per macro-edge (2^level)
 };
 
+// Row sums from the values val(q) at the stencil positions of the offsets in `valid`. All loads
+// are issued before the first sum: with the sum inside a branch per offset or micro-tet the
+// loads of a row waited for one another, and the passes over the surface DoFs and the row
+// tables were bound by that chain (variable coefficient, FP64, level 6 on 36 cells: 22 us per
+// interface colour, now 12; a row pass of the small levels 9.6 us alone, now 7.1).
+
+// constant operator: partial stencil st of the row's class, valid offsets `valid`. FP32 rows
+// read the positions of invalid offsets too (some position of the slab): 27 us an interface
+// colour at level 6 on 384 cells against 33 with the loads predicated; FP64 at level 7 on 48
+// cells: 24 against 20. The apply, whose surface part is bound by the number of gathers, keeps
+// the branches (AHEAD = false): 271 us at level 6 on 384 cells against 281.
+template < typename T, bool AHEAD = true, typename Val >
+__device__ __forceinline__ void rowConstant( const T* st, uint32_t valid, T& diag, T& off, Val&& val )
+{
+   if constexpr ( !AHEAD )
+   {
+      diag += st[0];
+#pragma unroll
+      for ( int q = 1; q < 15; ++q )
+         if ( valid & ( 1u << q ) )
+            off += st[q] * val( q );
+   }
+   else
+   {
+      T v[15];
+#pragma unroll
+      for ( int q = 1; q < 15; ++q )
+         v[q] = ( sizeof( T ) == 4 || ( valid & ( 1u << q ) ) ) ? val( q ) : T( 0 );
+      diag += st[0];
+#pragma unroll
+      for ( int q = 1; q < 15; ++q )
+      {
+         const T w = st[q];
+         if ( valid & ( 1u << q ) )
+            off += w * v[q];
+      }
+   }
+}
+
+// variable coefficient: the offsets `valid` and micro-tets validT around the point; at(q) is the slab position of
+// offset q. The weights of the 14 edges are collected over the tets (three per tet), the
+// off-diagonal sum takes one product per edge, and the diagonal is minus the sum of the
+// weights (the element matrices have zero row sums and are symmetric: one entry per pair).
+template < typename T, int VAR, typename Val, typename At >
+__device__ __forceinline__ void rowVariable( const OpDev< T >& op, int cell, uint32_t valid, uint32_t validT, T& diag,
+                                             T& off, Val&& val, At&& at )
+{
+   const T* kv = op.kap + size_t( cell ) * op.stride;
+   const T* K  = op.K + size_t( cell ) * 96;
+   T        kq[15], uq[15], a[15];
+#pragma unroll
+   for ( int q = 0; q < 15; ++q )
+   {
+      const bool in = valid & ( 1u << q );
+      if constexpr ( VAR == 1 )
+         kq[q] = in ? kv[at( q )] : T( 0 );
+      if ( q > 0 )
+         uq[q] = in ? val( q ) : T( 0 );
+      a[q] = 0;
+   }
+#pragma unroll
+   for ( int i = 0; i < 24; ++i )
+   {
+      const IncidentTet it = incidentTet( i );
+      T                 ks;
+      if constexpr ( VAR == 2 )
+         ks = op.kq[( size_t( cell ) * 6 + it.t ) * op.stride + at( it.q[0] )];
+      else
+         ks = kq[it.q[0]] + kq[it.q[1]] + kq[it.q[2]] + kq[it.q[3]];
+      ks = ( validT & ( 1u << i ) ) ? ks : T( 0 );
+#pragma unroll
+      for ( int j = 0; j < 4; ++j )
+         if ( j != it.k )
+            a[it.q[j]] += ks * K[it.t * 16 + ( j < it.k ? j * 4 + it.k : it.k * 4 + j )];
+   }
+#pragma unroll
+   for ( int q = 1; q < 15; ++q )
+   {
+      diag -= a[q];
+      if ( valid & ( 1u << q ) )
+         off += a[q] * uq[q];
+   }
+}
+
 // Partial row of the operator at closure point (x,y,z) of `cell`: the contributions
 // of the micro-tets of this cell only. u = the cell's slab. VAR (throughout the kernels):
 // 0 constant stencils, 1 variable coefficient from nodal values (OpDev::kap), 2 variable
 // coefficient integrated at quadrature points (OpDev::kq).
-template < typename T, int VAR >
+template < typename T, int VAR, bool AHEAD = true >
 __device__ __forceinline__ void partialRow( const OpDev< T >& op, const T* u, int cell, int W, int x, int y,
                                             int z, T& diag, T& off )
 {
@@ -367,40 +451,10 @@ __device__ __forceinline__ void partialRow( const OpDev< T >& op, const T* u, in
    if constexpr ( !VAR )
    {
       const T* st = op.st + ( size_t( cell ) * 16 + mask ) * 15;
-      diag += st[0];
-#pragma unroll
-      for ( int q = 1; q < 15; ++q )
-         if ( valid & ( 1u << q ) )
-            off += st[q] * u[pos[q]];
+      rowConstant< T, AHEAD >( st, valid, diag, off, [&]( int q ) { return u[pos[q]]; } );
    }
    else
-   {
-      const T*       kv    = op.kap + size_t( cell ) * op.stride;
-      const T*       kqc   = VAR == 2 ? op.kq + size_t( cell ) * 6 * op.stride : nullptr;
-      const T*       K     = op.K + size_t( cell ) * 96;
-      const uint32_t validT = kValidTets[mask];
-#pragma unroll
-      for ( int i = 0; i < 24; ++i )
-      {
-         const IncidentTet it = incidentTet( i );
-         if ( !( validT & ( 1u << i ) ) )
-            continue;
-         T ks;
-         if constexpr ( VAR == 2 )
-            ks = kqc[size_t( it.t ) * op.stride + pos[it.q[0]]];
-         else
-            ks = kv[pos[it.q[0]]] + kv[pos[it.q[1]]] + kv[pos[it.q[2]]] + kv[pos[it.q[3]]];
-         const T* Kr = K + it.t * 16 + it.k * 4;
-#pragma unroll
-         for ( int j = 0; j < 4; ++j )
-         {
-            if ( j == it.k )
-               diag += ks * Kr[j];
-            else
-               off += ks * Kr[j] * u[pos[it.q[j]]];
-         }
-      }
-   }
+      rowVariable< T, VAR >( op, cell, valid, kValidTets[mask], diag, off, [&]( int q ) { return u[pos[q]]; }, [&]( int q ) { return pos[q]; } );
 }
 
 } // namespace hyb

@@ -190,7 +190,7 @@ __device__ __forceinline__ T groupSum( T v, int G )
 }
 
 // Partial rows of the group's adjacent cells, summed over the group (all lanes get it).
-template < typename T, int VAR >
+template < typename T, int VAR, bool AHEAD = true >
 __device__ __forceinline__ void bdryRowGroup( const TopoDev& tp, const LevelDev& lv, const OpDev< T >& op, const T* u,
                                               const BdryPoint& p, const LaneTask& tk, bool active, T& diag, T& off )
 {
@@ -203,7 +203,7 @@ __device__ __forceinline__ void bdryRowGroup( const TopoDev& tp, const LevelDev&
       {
          int c, x, y, z;
          embeddingCoords( embAt( tp, p.kind, p.prim, e ), p.kind, lv.N, p.i, p.j, c, x, y, z );
-         partialRow< T, VAR >( op, u + size_t( c ) * lv.stride, c, lv.W, x, y, z, diag, off );
+         partialRow< T, VAR, AHEAD >( op, u + size_t( c ) * lv.stride, c, lv.W, x, y, z, diag, off );
       }
    }
    diag = groupSum( diag, tk.G );
@@ -765,10 +765,16 @@ __device__ __forceinline__ void rowPassBody( const RowPass& rp, const OpDev< T >
          B             = __ldg( p + 1 );
          C             = __ldg( p + 2 );
       }
-      const bool active = A.x >= 0 && ( ( A.z >> 16 ) & flag );
-      T          diag = 0, off = 0;
+      const bool   active = A.x >= 0 && ( ( A.z >> 16 ) & flag );
+      const size_t i      = active ? size_t( A.x ) + ( uint32_t( A.w ) & 0xffffu ) : 0;
+      T            diag = 0, off = 0, own = 0, bi = 0;
       if ( active )
       {
+         // the point's own value and right-hand side travel with the neighbours
+         if constexpr ( MODE != kRowInvDiag )
+            own = u[i];
+         if constexpr ( MODE == kRowSor || MODE == kRowResidual || MODE == kRowJacobi )
+            bi = b[i];
          const T*       uc    = u + A.x;
          const uint32_t valid = uint32_t( A.z ) & 0xffffu;
          // pos[q] of the row: 16-bit halves of A.w, B.xyzw, C.xyz
@@ -794,42 +800,12 @@ __device__ __forceinline__ void rowPassBody( const RowPass& rp, const OpDev< T >
                       int( uint32_t( C.w ) >> 16 ), kValidTets[( A.y / 15 ) & 15], spos, diag, off );
          }
          else if constexpr ( !VAR )
-         {
-            const T* w = op.st + A.y;
-            diag += w[0];
-#pragma unroll
-            for ( int q = 1; q < 15; ++q )
-               if ( valid & ( 1u << q ) )
-                  off += w[q] * uc[pos( q )];
-         }
+            rowConstant( op.st + A.y, valid, diag, off, [&]( int q ) { return uc[pos( q )]; } );
          else
          {
-            const int      cls    = ( A.y / 15 ) & 15, cell = A.y / 240;
-            const T*       kv     = op.kap + A.x;
-            const T*       kqc    = VAR == 2 ? op.kq + size_t( cell ) * 6 * op.stride : nullptr;
-            const T*       K      = op.K + size_t( cell ) * 96;
-            const uint32_t validT = kValidTets[cls];
-#pragma unroll
-            for ( int i = 0; i < 24; ++i )
-            {
-               const IncidentTet it = incidentTet( i );
-               if ( !( validT & ( 1u << i ) ) )
-                  continue;
-               T ks;
-               if constexpr ( VAR == 2 )
-                  ks = kqc[size_t( it.t ) * op.stride + pos( it.q[0] )];
-               else
-                  ks = kv[pos( it.q[0] )] + kv[pos( it.q[1] )] + kv[pos( it.q[2] )] + kv[pos( it.q[3] )];
-               const T* Kr = K + it.t * 16 + it.k * 4;
-#pragma unroll
-               for ( int j = 0; j < 4; ++j )
-               {
-                  if ( j == it.k )
-                     diag += ks * Kr[j];
-                  else
-                     off += ks * Kr[j] * uc[pos( it.q[j] )];
-               }
-            }
+            // base = cell * stride
+            const int cls = ( A.y / 15 ) & 15, cell = A.y / 240;
+            rowVariable< T, VAR >( op, cell, valid, kValidTets[cls], diag, off, [&]( int q ) { return uc[pos( q )]; }, pos );
          }
       }
       const int G = gt < rp.b1 ? 32 : gt < rp.b2 ? 8 : gt < rp.b3 ? 2 : 1;
@@ -837,19 +813,18 @@ __device__ __forceinline__ void rowPassBody( const RowPass& rp, const OpDev< T >
       off         = groupSum( off, G );
       if ( !active )
          continue;
-      const size_t i = size_t( A.x ) + ( uint32_t( A.w ) & 0xffffu );
       if constexpr ( MODE == kRowSor )
-         u[i] = ( T( 1 ) - relax ) * u[i] + relax * ( b[i] - off ) / diag;
+         u[i] = ( T( 1 ) - relax ) * own + relax * ( bi - off ) / diag;
       else if constexpr ( MODE == kRowResidual )
-         r[i] = b[i] - ( diag * u[i] + off );
+         r[i] = bi - ( diag * own + off );
       else if constexpr ( MODE == kRowApplyAdd )
-         r[i] += diag * u[i] + off;
+         r[i] += diag * own + off;
       else if constexpr ( MODE == kRowJacobi )
-         r[i] = u[i] + relax * ( b[i] - off - diag * u[i] ) / diag;
+         r[i] = own + relax * ( bi - off - diag * own ) / diag;
       else if constexpr ( MODE == kRowInvDiag )
          r[i] = T( 1 ) / diag;
       else
-         r[i] = diag * u[i] + off;
+         r[i] = diag * own + off;
    }
 }
 
@@ -1028,19 +1003,25 @@ __device__ __forceinline__ void applyBody( Blk vb, TopoDev tp, LevelDev lv, OpDe
       const LaneTask  tk     = laneTask( tp, lv, bl, gt );
       const BdryPoint p      = decodeBdry( tp, lv, tk.t );
       const bool      active = tk.valid && ( primBc( tp, p.kind, p.prim ) & flag );
-      T               diag, off;
-      bdryRowGroup< T, VAR >( tp, lv, op, src, p, tk, active, diag, off );
+      T               diag, off, own = 0, b = 0;
+      if ( active )
+      {
+         const size_t r0 = bdryReplica< T >( tp, lv, p, 0 );
+         own             = src[r0];
+         if constexpr ( MODE != kReplace )
+            b = MODE == kAdd ? dst[r0] : rhs[r0];
+      }
+      bdryRowGroup< T, VAR, false >( tp, lv, op, src, p, tk, active, diag, off );
       if ( !active )
          continue;
-      const size_t r0 = bdryReplica< T >( tp, lv, p, 0 );
-      const T      ax = diag * src[r0] + off;
-      T            v;
+      const T ax = diag * own + off;
+      T       v;
       if constexpr ( MODE == kReplace )
          v = ax;
       else if constexpr ( MODE == kAdd )
-         v = dst[r0] + ax;
+         v = b + ax;
       else
-         v = rhs[r0] - ax;
+         v = b - ax;
       if constexpr ( MODE == kResidualNorm )
       {
          // the first embedding's lane counts the DoF once; every replica gets float(r)
@@ -1111,20 +1092,27 @@ __device__ __forceinline__ void sorIfaceBody( Blk vb, TopoDev tp, LevelDev lv, O
       const LaneTask  tk     = laneTask( tp, lv, bl, gt );
       const BdryPoint p      = decodeBdry( tp, lv, tk.t );
       const bool      active = tk.valid && ( primBc( tp, p.kind, p.prim ) & flag );
-      T               diag, off;
+      T               diag, off, own = 0, b = 0;
+      if ( active )
+      {
+         const size_t r0 = bdryReplica< T >( tp, lv, p, 0 );
+         own             = u[r0];
+         b               = rhs[r0];
+      }
       bdryRowGroup< T, VAR >( tp, lv, op, u, p, tk, active, diag, off );
       if ( !active )
          continue;
-      const size_t r0 = bdryReplica< T >( tp, lv, p, 0 );
-      const T      v  = ( T( 1 ) - relax ) * u[r0] + relax * ( rhs[r0] - off ) / diag;
+      const T v = ( T( 1 ) - relax ) * own + relax * ( b - off ) / diag;
       // all lanes of the group read u[r0] before any replica is written
       __syncwarp( __activemask() );
       bdryWriteGroup( tp, lv, p, tk, u, v );
    }
 }
 
+// (constant operator, FP64 at level 7 on 48 cells: 26 us a colour with eight resident blocks, 20
+// with six and no spills; FP32 at level 6 on 384 cells: 27 with eight, 37 with six)
 template < typename T, int VAR >
-__global__ void __launch_bounds__( 128, VAR ? 4 : 8 ) k_sor_iface( TopoDev tp, LevelDev lv, OpDev< T > op, T* __restrict__ u,
+__global__ void __launch_bounds__( 128, VAR ? 4 : ( sizeof( T ) == 8 ? 6 : 8 ) ) k_sor_iface( TopoDev tp, LevelDev lv, OpDev< T > op, T* __restrict__ u,
                                                       const T* __restrict__ rhs, T relax, int flag, BdryLists bl )
 {
    HYB_PDL_PROLOGUE();
