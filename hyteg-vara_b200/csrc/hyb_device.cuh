@@ -144,6 +144,37 @@ __constant__ const uint32_t kValidTets[16] = { 0xffffff, 0xe324ae, 0x9e4a4d, 0x8
                                                0x040809, 0x000008, 0x381377, 0x200026, 0x180245, 0x000004,
                                                0x000113, 0x000002, 0x000001, 0x000000 };
 
+// The tets around the edge from a point to its neighbour q: their other vertices form a ring of
+// six or four, symmetric about the edge's midpoint. ringVertex( q, i ) lists them as pairs of
+// opposite ones (i = 0, 1 the first pair; offsets from the point), ringPairs( q ) counts the
+// pairs. Opposite ring vertices see element matrices of point-reflected, hence equal, tets:
+// the edge's weight is sum_j beta_j ( k_v + k_v' + k_p + k_q ) over the pairs, with k the
+// nodal coefficient and beta_j the sum of the edge's entries in the two tets that hold v. The
+// edges q and -q have the same beta; ringBeta( b, i ) are the two entries (t * 16 + a * 4 + b)
+// that make up beta number b, numbered from ringFirst( q ).
+__host__ __device__ constexpr int ringVertex( int q, int i )
+{
+   constexpr int t[15][6] = { { 0, 0, 0, 0, 0, 0 },    { 3, 8, 5, 10, 12, 14 }, { 7, 4, 9, 6, 13, 11 },  { 1, 7, 5, 12, 0, 0 },
+                              { 8, 2, 11, 6, 0, 0 },   { 1, 9, 3, 11, 7, 14 },  { 10, 2, 12, 4, 13, 8 }, { 2, 3, 5, 13, 9, 12 },
+                              { 4, 1, 14, 6, 11, 10 }, { 2, 5, 7, 11, 0, 0 },   { 6, 1, 12, 8, 0, 0 },   { 2, 14, 4, 5, 8, 9 },
+                              { 13, 1, 6, 3, 10, 7 },  { 2, 12, 6, 7, 0, 0 },   { 11, 1, 8, 5, 0, 0 } };
+   return t[q][i];
+}
+__host__ __device__ constexpr int ringPairs( int q ) { return q == 3 || q == 4 || q == 9 || q == 10 || q >= 13 ? 2 : 3; }
+__host__ __device__ constexpr int ringFirst( int q )
+{
+   constexpr int t[7] = { 0, 3, 5, 8, 11, 13, 16 };
+   return t[( q - 1 ) / 2];
+}
+constexpr int                     kRingBetas = 18;
+__host__ __device__ constexpr int ringBeta( int b, int i )
+{
+   constexpr int t[kRingBetas][2] = { { 1, 66 },  { 1, 81 },  { 43, 66 }, { 2, 70 },  { 2, 17 },  { 3, 83 },
+                                      { 3, 19 },  { 19, 34 }, { 6, 65 },  { 18, 33 }, { 6, 33 },  { 7, 87 },
+                                      { 7, 35 },  { 23, 86 }, { 11, 23 }, { 11, 39 }, { 38, 67 }, { 27, 38 } };
+   return t[b][i];
+}
+
 // The 24 micro-tets incident to a micro-vertex: micro-cell type t (WHITE_UP, BLUE_UP,
 // GREEN_UP, WHITE_DOWN, BLUE_DOWN, GREEN_DOWN of src/hyteg/volumedofspace/CellDoFIndexing.hpp:
 // 155-198), the vertex's role k in it, and the stencil offset of each of its 4 vertices.
@@ -350,15 +381,30 @@ struct OpDev
 // tables were bound by that chain (variable coefficient, FP64, level 6 on 36 cells: 22 us per
 // interface colour, now 12; a row pass of the small levels 9.6 us alone, now 7.1).
 
-// constant operator: partial stencil st of the row's class, valid offsets `valid`. FP32 rows
-// read the positions of invalid offsets too (some position of the slab): 27 us an interface
-// colour at level 6 on 384 cells against 33 with the loads predicated; FP64 at level 7 on 48
-// cells: 24 against 20. The apply, whose surface part is bound by the number of gathers, keeps
-// the branches (AHEAD = false): 271 us at level 6 on 384 cells against 281.
-template < typename T, bool AHEAD = true, typename Val >
+// How the constant operator's row reads its values: the loads of the valid offsets ahead of the
+// sums, those of all offsets (the position of an invalid one is some position of the slab),
+// or each load in its term's branch. FP32 surface rows read all: 27 us an interface colour at
+// level 6 on 384 cells against 33 for the valid ones; FP64 the valid ones: 20 us at level 7 on
+// 48 cells against 24, and an FP64 cycle on 6 cells, levels 0..5, whose row tables' passes
+// dominate: 497 us against 541. The apply, whose surface part is bound by the number of
+// gathers, keeps the branches: 271 us at level 6 on 384 cells against 281.
+enum RowLoads : int
+{
+   kRowValid  = 0,
+   kRowAll    = 1,
+   kRowBranch = 2
+};
+template < typename T >
+__host__ __device__ constexpr int rowLoads()
+{
+   return sizeof( T ) == 4 ? kRowAll : kRowValid;
+}
+
+// constant operator: partial stencil st of the row's class, valid offsets `valid`
+template < typename T, int LOADS, typename Val >
 __device__ __forceinline__ void rowConstant( const T* st, uint32_t valid, T& diag, T& off, Val&& val )
 {
-   if constexpr ( !AHEAD )
+   if constexpr ( LOADS == kRowBranch )
    {
       diag += st[0];
 #pragma unroll
@@ -371,7 +417,7 @@ __device__ __forceinline__ void rowConstant( const T* st, uint32_t valid, T& dia
       T v[15];
 #pragma unroll
       for ( int q = 1; q < 15; ++q )
-         v[q] = ( sizeof( T ) == 4 || ( valid & ( 1u << q ) ) ) ? val( q ) : T( 0 );
+         v[q] = ( LOADS == kRowAll || ( valid & ( 1u << q ) ) ) ? val( q ) : T( 0 );
       diag += st[0];
 #pragma unroll
       for ( int q = 1; q < 15; ++q )
@@ -432,7 +478,7 @@ __device__ __forceinline__ void rowVariable( const OpDev< T >& op, int cell, uin
 // of the micro-tets of this cell only. u = the cell's slab. VAR (throughout the kernels):
 // 0 constant stencils, 1 variable coefficient from nodal values (OpDev::kap), 2 variable
 // coefficient integrated at quadrature points (OpDev::kq).
-template < typename T, int VAR, bool AHEAD = true >
+template < typename T, int VAR, int LOADS = rowLoads< T >() >
 __device__ __forceinline__ void partialRow( const OpDev< T >& op, const T* u, int cell, int W, int x, int y,
                                             int z, T& diag, T& off )
 {
@@ -451,7 +497,7 @@ __device__ __forceinline__ void partialRow( const OpDev< T >& op, const T* u, in
    if constexpr ( !VAR )
    {
       const T* st = op.st + ( size_t( cell ) * 16 + mask ) * 15;
-      rowConstant< T, AHEAD >( st, valid, diag, off, [&]( int q ) { return u[pos[q]]; } );
+      rowConstant< T, LOADS >( st, valid, diag, off, [&]( int q ) { return u[pos[q]]; } );
    }
    else
       rowVariable< T, VAR >( op, cell, valid, kValidTets[mask], diag, off, [&]( int q ) { return u[pos[q]]; }, [&]( int q ) { return pos[q]; } );

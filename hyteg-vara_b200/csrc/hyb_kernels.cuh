@@ -190,7 +190,7 @@ __device__ __forceinline__ T groupSum( T v, int G )
 }
 
 // Partial rows of the group's adjacent cells, summed over the group (all lanes get it).
-template < typename T, int VAR, bool AHEAD = true >
+template < typename T, int VAR, int LOADS = rowLoads< T >() >
 __device__ __forceinline__ void bdryRowGroup( const TopoDev& tp, const LevelDev& lv, const OpDev< T >& op, const T* u,
                                               const BdryPoint& p, const LaneTask& tk, bool active, T& diag, T& off )
 {
@@ -203,7 +203,7 @@ __device__ __forceinline__ void bdryRowGroup( const TopoDev& tp, const LevelDev&
       {
          int c, x, y, z;
          embeddingCoords( embAt( tp, p.kind, p.prim, e ), p.kind, lv.N, p.i, p.j, c, x, y, z );
-         partialRow< T, VAR, AHEAD >( op, u + size_t( c ) * lv.stride, c, lv.W, x, y, z, diag, off );
+         partialRow< T, VAR, LOADS >( op, u + size_t( c ) * lv.stride, c, lv.W, x, y, z, diag, off );
       }
    }
    diag = groupSum( diag, tk.G );
@@ -241,8 +241,10 @@ template < typename T, int VAR >
 struct InteriorOp
 {
    T w[15];       // constant operator: the class-0 stencil of the cell
-   T ku[36];      // variable operator: the 6 off-diagonal entries (pairs 01 02 03 12 13 23)
-                  // of each of the cell's 6 micro-tet matrices, held in registers
+   T ku[36];      // variable operator at quadrature points: the 6 off-diagonal entries (pairs 01
+                  // 02 03 12 13 23) of each of the cell's 6 micro-tet matrices
+   T beta[kRingBetas], alpha[7]; // variable operator, nodal k: the cell's edge weights (ringBeta)
+                                 // and their sums per edge direction
    const T* kv;   // variable operator: nodal k slab of the cell
    const T* kqc;  // variable operator at quadrature points: the cell's 6 micro-tet factor slabs
    int      kqs;  // their stride
@@ -266,13 +268,28 @@ struct InteriorOp
       else
       {
          const T* K = op.K + size_t( cell ) * 96;
+         if constexpr ( VAR == 1 )
+         {
 #pragma unroll
-         for ( int t = 0; t < 6; ++t )
+            for ( int b = 0; b < kRingBetas; ++b )
+               beta[b] = K[ringBeta( b, 0 )] + K[ringBeta( b, 1 )];
 #pragma unroll
-            for ( int a = 0; a < 4; ++a )
+            for ( int d = 0; d < 7; ++d )
+            {
+               const int f = ringFirst( 2 * d + 1 );
+               alpha[d]    = beta[f] + beta[f + 1] + ( ringPairs( 2 * d + 1 ) == 3 ? beta[f + 2] : T( 0 ) );
+            }
+         }
+         else
+         {
 #pragma unroll
-               for ( int b = a + 1; b < 4; ++b )
-                  ku[6 * t + pairIdx( a, b )] = K[t * 16 + a * 4 + b];
+            for ( int t = 0; t < 6; ++t )
+#pragma unroll
+               for ( int a = 0; a < 4; ++a )
+#pragma unroll
+                  for ( int b = a + 1; b < 4; ++b )
+                     ku[6 * t + pairIdx( a, b )] = K[t * 16 + a * 4 + b];
+         }
          kv  = op.kap + size_t( cell ) * op.stride;
          kqc = VAR == 2 ? op.kq + size_t( cell ) * 6 * op.stride : nullptr;
          kqs = op.stride;
@@ -322,6 +339,11 @@ struct InteriorOp
       }
       else
       {
+         // the weight of each of the 14 edges from the coefficient at its ends and on its ring
+         // (8 or 6 operations), then one product per edge; zero row sums give the diagonal.
+         // Summing over the 24 tets instead takes 240 operations a row, this 128. The passes are
+         // bound by the reads through L1, so it gives little: 20.9 -> 20.0 us an FP64 interior
+         // colour at level 6 on 36 cells, weights read once per strip of batches included.
          T kq[15], uq[15];
 #pragma unroll
          for ( int q = 0; q < 15; ++q )
@@ -329,25 +351,17 @@ struct InteriorOp
             kq[q] = kv[no.d[q] + g];
             uq[q] = u[no.d[q] + g];
          }
-         // element matrices of P1 stiffness have zero row sums, so the diagonal entry is
-         // minus the sum of the row's off-diagonal entries (symmetric: one value per pair)
          T d = 0, s = 0;
 #pragma unroll
-         for ( int i = 0; i < 24; ++i )
+         for ( int q = 1; q < 15; ++q )
          {
-            const IncidentTet it = incidentTet( i );
-            const T ks = kq[it.q[0]] + kq[it.q[1]] + kq[it.q[2]] + kq[it.q[3]];
-            T       rowsum = 0, acc = 0;
+            T a = alpha[( q - 1 ) / 2] * ( kq[0] + kq[q] );
 #pragma unroll
-            for ( int j = 0; j < 4; ++j )
-               if ( j != it.k )
-               {
-                  const T c = ku[6 * it.t + pairIdx( it.k, j )];
-                  rowsum += c;
-                  acc += c * uq[it.q[j]];
-               }
-            d -= ks * rowsum;
-            s += ks * acc;
+            for ( int j = 0; j < 3; ++j )
+               if ( j < ringPairs( q ) )
+                  a += beta[ringFirst( q ) + j] * ( kq[ringVertex( q, 2 * j )] + kq[ringVertex( q, 2 * j + 1 )] );
+            d -= a;
+            s += a * uq[q];
          }
          diag = d;
          off  = s;
@@ -415,6 +429,11 @@ __host__ __device__ constexpr int interiorBatch()
 {
    return VAR ? 1 : ( sizeof( T ) == 8 ? 3 : 2 );
 }
+
+// consecutive interior batches a warp takes per block step at most (measured at level 7
+// on B200: 1 -> 435 us, 2 -> 428, 4 -> 413, 8 -> 422, 16 -> 476 us per FP64 sweep; on
+// smaller levels long strips leave blocks idle, so the strip shrinks with the work)
+constexpr int kInteriorStrip = 4;
 
 // The K table entries i0 + 32 k of a point table. Entries past the end are clamped to the
 // last one, so every read stays in bounds; valid[k] tells the caller not to store them.
@@ -800,7 +819,7 @@ __device__ __forceinline__ void rowPassBody( const RowPass& rp, const OpDev< T >
                       int( uint32_t( C.w ) >> 16 ), kValidTets[( A.y / 15 ) & 15], spos, diag, off );
          }
          else if constexpr ( !VAR )
-            rowConstant( op.st + A.y, valid, diag, off, [&]( int q ) { return uc[pos( q )]; } );
+            rowConstant< T, rowLoads< T >() >( op.st + A.y, valid, diag, off, [&]( int q ) { return uc[pos( q )]; } );
          else
          {
             // base = cell * stride
@@ -957,13 +976,18 @@ __device__ __forceinline__ void applyBody( Blk vb, TopoDev tp, LevelDev lv, OpDe
    {
       constexpr int K       = interiorBatch< T, VAR >();
       const int     nChunks = ( lv.nPts + 32 * K - 1 ) / ( 32 * K );
-      HYB_CELL_LOOP( nChunks )
+      // strips as in sorInteriorBody: the cell's weights serve several batches of a warp
+      const int            strip = max( 1, min( kInteriorStrip, tp.nC * nChunks / ( nCellBlocks * int( blockDim.x >> 5 ) ) ) );
+      InteriorOp< T, VAR > io;
+      int                  loaded = -1;
+      HYB_CELL_LOOP_STRIP( nChunks, strip )
       {
          const int     cell = it_ / nChunks;
          PointBatch< K > pb;
          pb.load( lv.pts, lv.blk, lv.nPts, ( it_ - cell * nChunks ) * 32 * K + int( threadIdx.x & 31 ) );
-         InteriorOp< T, VAR > io;
-         io.load( op, cell );
+         if ( cell != loaded )
+            io.load( op, cell );
+         loaded = cell;
          const size_t co = size_t( cell ) * lv.stride;
          const T* su = src + co;
          T ax[K];
@@ -1011,7 +1035,7 @@ __device__ __forceinline__ void applyBody( Blk vb, TopoDev tp, LevelDev lv, OpDe
          if constexpr ( MODE != kReplace )
             b = MODE == kAdd ? dst[r0] : rhs[r0];
       }
-      bdryRowGroup< T, VAR, false >( tp, lv, op, src, p, tk, active, diag, off );
+      bdryRowGroup< T, VAR, kRowBranch >( tp, lv, op, src, p, tk, active, diag, off );
       if ( !active )
          continue;
       const T ax = diag * own + off;
@@ -1077,10 +1101,6 @@ __global__ void __launch_bounds__( 128, VAR ? 3 : 8 ) k_residual_norm( TopoDev t
 // cell interiors. No two DoFs of one pass are coupled.
 // ---------------------------------------------------------------------------
 constexpr int kInteriorColours = 4;
-// consecutive interior batches a warp takes per block step at most (measured at level 7
-// on B200: 1 -> 435 us, 2 -> 428, 4 -> 413, 8 -> 422, 16 -> 476 us per FP64 sweep; on
-// smaller levels long strips leave blocks idle, so the strip shrinks with the work)
-constexpr int kInteriorStrip = 4;
 
 template < typename T, int VAR >
 __device__ __forceinline__ void sorIfaceBody( Blk vb, TopoDev tp, LevelDev lv, OpDev< T > op, T* u,
@@ -1133,14 +1153,17 @@ __device__ __forceinline__ void sorInteriorBody( Blk vb, TopoDev tp, LevelDev lv
    const int      nChunks = ( nPts + 32 * K - 1 ) / ( 32 * K );
    // strips only while every warp of the grid still gets at least one strip
    const int strip = max( 1, min( kInteriorStrip, tp.nC * nChunks / ( nCellBlocks * int( blockDim.x >> 5 ) ) ) );
+   InteriorOp< T, VAR > io;
+   int                  loaded = -1;
    HYB_CELL_LOOP_STRIP( nChunks, strip )
    {
       const int       item = ( colour & 1 ) ? nItems_ - 1 - it_ : it_;
       const int       cell = item / nChunks;
       PointBatch< K > pb;
       pb.load( pts, lv.blk, nPts, ( item - cell * nChunks ) * 32 * K + int( threadIdx.x & 31 ) );
-      InteriorOp< T, VAR > io;
-      io.load( op, cell );
+      if ( cell != loaded )
+         io.load( op, cell );
+      loaded = cell;
       T*       uc = u + size_t( cell ) * lv.stride;
       const T* bc = rhs + size_t( cell ) * lv.stride;
       // constant operator: the diagonal is the cell's stencil centre, one reciprocal per batch
@@ -1166,8 +1189,10 @@ __device__ __forceinline__ void sorInteriorBody( Blk vb, TopoDev tp, LevelDev lv
    }
 }
 
+// (nodal coefficient: registers for four resident blocks in FP64 and six in FP32 without spills
+// to speak of)
 template < typename T, int VAR >
-__global__ void __launch_bounds__( 128 ) k_sor_interior( TopoDev tp, LevelDev lv, OpDev< T > op, T* __restrict__ u,
+__global__ void __launch_bounds__( 128, VAR == 1 ? ( sizeof( T ) == 8 ? 4 : 6 ) : 1 ) k_sor_interior( TopoDev tp, LevelDev lv, OpDev< T > op, T* __restrict__ u,
                                                          const T* __restrict__ rhs, T relax, int colour, int begin,
                                                          int nPts, int nCellBlocks )
 {

@@ -22,7 +22,7 @@ struct LevelHost
    std::unique_ptr< RowTables > rows; // built on first use (ensureRows)
    bool                         rowsTried = false;
    std::unique_ptr< RowTables > blendRows; // full rows for blending operators (ensureBlendRows)
-   DevBuf< int32_t >  seg, xyz, linPos, blk, blkXYZ, pts, ptsC, quads, rowYZ;
+   DevBuf< int32_t >  seg, xyz, blk, blkXYZ, pts, ptsC, quads, rowYZ; // xyz: then linPos
    DevBuf< int32_t >  lexCell, lexCellOff, lexFace, lexFaceOff; // LevelDev::lex* (ensureLex)
    DevBuf< int4 >     lexCellNbr;                                  // LevelDev::lexCellNbr
    DevBuf< int32_t >  lexOfPts, lexSidx;                           // LevelDev::lexOfPts, lexSidx
@@ -342,13 +342,13 @@ void buildStorage( Storage& s, const std::vector< std::array< double, 3 > >& V, 
             for ( int x = 1; x + y + z <= d.N - 1; ++x )
                linPos.push_back( sidx( d.W, x, y, z ) );
       require( int( linPos.size() ) == d.nIntCell, "interior point count" );
-      lh->linPos.upload( linPos );
-      d.linPos = lh->linPos.p;
       lh->seg.upload( seg );
+      xyz.insert( xyz.end(), linPos.begin(), linPos.end() ); // one allocation
       lh->xyz.upload( xyz );
       d.nSeg = int( seg.size() );
       d.seg  = lh->seg.p;
       d.xyz  = lh->xyz.p;
+      d.linPos = lh->xyz.p + d.S;
       // grids: the loops are grid-stride, so a few resident blocks per SM suffice
       auto grid = [&]( long work, int perBlock, int perSM ) {
          return int( std::max< long >( 0, std::min< long >( ( work + perBlock - 1 ) / perBlock, long( s.numSMs ) * perSM ) ) );
