@@ -5,15 +5,16 @@
 import os
 import subprocess
 import sys
+import tempfile
 
 HERE = os.path.dirname(os.path.abspath(__file__))
-SRC = [os.path.join(HERE, "csrc", f) for f in ("hyb_capi.cu", "topology.cpp")]
-DEPS = SRC + [os.path.join(HERE, "csrc", f) for f in ("hyb_device.cuh", "hyb_kernels.cuh", "hyb_program.cuh", "hyb_storage.inl", "hyb_launch.inl", "hyb_gmg.inl", "hyb_server.inl", "topology.hpp")] + \
+SRC = [os.path.join(HERE, "csrc", f) for f in ("hyb_capi.cu", "hyb_surface.cu", "topology.cpp")]
+DEPS = SRC + [os.path.join(HERE, "csrc", f) for f in ("hyb_device.cuh", "hyb_kernels.cuh", "hyb_program.cuh", "hyb_storage.inl", "hyb_launch.inl", "hyb_gmg.inl", "hyb_server.inl", "hyb_surface.hpp", "hyb_surface_dofs.cuh", "topology.hpp")] + \
     [os.path.join(os.path.dirname(HERE), "include", "hyteg_b200.h")]
 OUT = os.path.join(HERE, "libhyteg_b200.so")
 NVCC = os.environ.get("NVCC", "/usr/local/cuda/bin/nvcc")
 FLAGS = ["-gencode", "arch=compute_100a,code=sm_100a", "-O3", "-lineinfo", "-std=c++17", "-Xcompiler", "-fPIC",
-         "-shared", "-Xptxas", "-warn-spills"]
+         "-Xptxas", "-warn-spills"]
 
 
 def up_to_date():
@@ -26,8 +27,14 @@ def up_to_date():
 def build(force=False, verbose=False):
     if not force and up_to_date():
         return OUT
-    cmd = [NVCC] + FLAGS + (["-Xptxas", "-v"] if verbose else []) + ["-o", OUT] + SRC
-    subprocess.run(cmd, check=True)
+    flags = FLAGS + (["-Xptxas", "-v"] if verbose else [])
+    with tempfile.TemporaryDirectory() as tmp:
+        # the translation units compile side by side
+        objs = [os.path.join(tmp, os.path.basename(f) + ".o") for f in SRC]
+        jobs = [subprocess.Popen([NVCC] + flags + ["-c", "-o", o, f]) for f, o in zip(SRC, objs)]
+        if any([j.wait() for j in jobs]):
+            raise subprocess.CalledProcessError(1, NVCC)
+        subprocess.run([NVCC, "-shared"] + FLAGS + ["-o", OUT] + objs, check=True)
     return OUT
 
 

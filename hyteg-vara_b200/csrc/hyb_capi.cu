@@ -18,6 +18,7 @@
 #include "../../include/hyteg_b200.h"
 #include "hyb_kernels.cuh"
 #include "hyb_program.cuh"
+#include "hyb_surface.hpp"
 #include "topology.hpp"
 
 namespace hyb {

@@ -478,9 +478,10 @@ __device__ __forceinline__ void rowVariable( const OpDev< T >& op, int cell, uin
 // of the micro-tets of this cell only. u = the cell's slab. VAR (throughout the kernels):
 // 0 constant stencils, 1 variable coefficient from nodal values (OpDev::kap), 2 variable
 // coefficient integrated at quadrature points (OpDev::kq).
-template < typename T, int VAR, int LOADS = rowLoads< T >() >
-__device__ __forceinline__ void partialRow( const OpDev< T >& op, const T* u, int cell, int W, int x, int y,
-                                            int z, T& diag, T& off )
+// U: const T*, or a type that reads the values another way.
+template < typename T, int VAR, int LOADS = rowLoads< T >(), typename U >
+__device__ __forceinline__ void partialRow( const OpDev< T >& op, U u, int cell, int W, int x, int y, int z, T& diag,
+                                            T& off )
 {
    const int         N     = W - 1;
    const int         mask  = classMask( N, x, y, z );

@@ -386,6 +386,20 @@ static const int kFusedInteriorMaxPoints = [] {
    return e ? std::atoi( e ) : 4096;
 }();
 
+// Whether the interface colours of level l run as one cooperative launch (hyb_surface.cu): from
+// this many surface DoFs on (HYB_SURFACE_MIN_DOFS overrides it). At level 6 on 48 cells (0.25 M)
+// a sweep's six launches take 40 us and the one 61; at level 7 on 48 cells (1 M) 130 against
+// 100, at level 6 on 384 cells (1.8 M, FP32) 165 against 130.
+constexpr long kSurfaceMinDofs = 500000;
+template < typename T >
+bool surfaceSor( const Operator& op, int l, int flag )
+{
+   static const long  minDofs = envLong( "HYB_SURFACE_MIN_DOFS", kSurfaceMinDofs );
+   const LevelHost&   L       = op.st->L( l );
+   return varKind( op ) == 0 && !op.blend && flag == ( HYB_INNER | HYB_NEUMANN ) && L.surface.nBlocks > 0 &&
+          L.dev.nBdry >= minDofs && surfaceSmem( L.surface, sizeof( T ) ) <= kSurfaceMaxSmem;
+}
+
 template < typename T >
 void launchSor( const Operator& op, int l, T* u, const T* rhs, T relax, int flag, cudaStream_t stream, bool backwards = false )
 {
@@ -488,17 +502,25 @@ void launchSor( const Operator& op, int l, T* u, const T* rhs, T relax, int flag
    };
    // forward: surface colours 0..m-1, then the interior colours 0..3; backwards (the
    // multicolour smooth_sor_backwards, P1Operator.hpp:385-400): the same passes reversed
+   auto interfaces = [&]() {
+      if ( surfaceSor< T >( op, l, flag ) )
+      {
+         HYB_CUDA( launchSurfaceSor< T >( s.td, L.dev, L.surface, od, u, rhs, relax, backwards, stream ) );
+         HYB_CHECK_LAUNCH();
+         return;
+      }
+      for ( int c = 0; c < s.td.m; ++c )
+         iface( backwards ? s.td.m - 1 - c : c );
+   };
    if ( !backwards )
    {
-      for ( int c = 0; c < s.td.m; ++c )
-         iface( c );
+      interfaces();
       interior();
    }
    else
    {
       interior();
-      for ( int c = s.td.m - 1; c >= 0; --c )
-         iface( c );
+      interfaces();
    }
 }
 

@@ -28,6 +28,9 @@ struct LevelHost
    DevBuf< int32_t >  lexOfPts, lexSidx;                           // LevelDev::lexOfPts, lexSidx
    bool               lexBuilt = false;
    DevBuf< int4 >     pro; // prolongation table (LevelDev::pro)
+   SurfaceDev         surface{};         // macro-face tiles of the one-launch interface passes (nBlocks 0: none)
+   DevBuf< FaceTile > faceTiles;
+   DevBuf< int32_t >  faceTileOff;
    DevBuf< int32_t >  colourList;        // surface-DoF indices grouped by SOR colour
    std::vector< int > colourOff;         // per colour: offset, #vertex, #edge, #face DoFs
    int                cellBlocks   = 0;  // grid of the cell-interior row-segment loops
@@ -105,6 +108,69 @@ struct Storage
 };
 
 inline int stridePad( int s ) { return ( s + 31 ) / 32 * 32; }
+
+// Deal the inner macro-faces of a level to blocks (SurfaceDev, hyb_surface.cu). A face is cut
+// into `parts` row ranges of about equal size, as few as leave the fullest block the least
+// work: 72 faces on 148 SMs are cut in two, 672 are not cut.
+void buildSurface( const Storage& s, LevelHost& lh )
+{
+   const LevelDev& d  = lh.dev;
+   SurfaceDev&     sf = lh.surface;
+   sf                 = SurfaceDev{};
+   std::vector< int > faces;
+   for ( size_t f = 0; f < s.topo.F.size(); ++f )
+      if ( s.topo.fBc[f] == kInner )
+         faces.push_back( int( f ) );
+   // the point coordinates of a list entry take 7 bits each
+   if ( d.N > 128 || d.N < 8 || faces.empty() || s.topo.colours > kSurfaceMaxColours )
+      return;
+   const long nF = long( faces.size() ), nB = s.numSMs;
+   int        parts = 1;
+   double     best  = 1e30;
+   for ( int p = 1; p <= 4 && ( p == 1 || nF < nB ); ++p )
+   {
+      const double load = double( ( nF * p + nB - 1 ) / nB ) / p;
+      if ( load < best - 1e-9 )
+         best = load, parts = p;
+   }
+   const long nT = nF * parts;
+   sf.nBlocks    = int( std::min( nB, nT ) );
+   auto first    = [&]( int j ) { return ( j - 1 ) * ( d.N - 1 ) - ( j - 1 ) * j / 2; }; // face index of (1, j)
+   std::vector< FaceTile > tiles;
+   for ( int f : faces )
+      for ( int p = 0, j = 1; p < parts; ++p )
+      {
+         int e = j;
+         while ( e < d.N - 1 && ( p == parts - 1 || long( first( e ) ) * parts < long( p + 1 ) * d.nIntFace ) )
+            ++e;
+         tiles.push_back( FaceTile{ f, j, e } );
+         j = e;
+      }
+   std::vector< int32_t > off( 1, 0 );
+   for ( int b = 0; b < sf.nBlocks; ++b )
+   {
+      off.push_back( int32_t( nT * ( b + 1 ) / sf.nBlocks ) );
+      int held = 0;
+      for ( int t = off[size_t( b )]; t < off[size_t( b ) + 1]; ++t )
+         held += first( std::min( tiles[size_t( t )].jb + 1, d.N - 1 ) ) - first( std::max( tiles[size_t( t )].ja - 1, 1 ) );
+      sf.most  = std::max( sf.most, ( held + 7 ) / 8 * 8 );
+      sf.tiles = std::max( sf.tiles, off[size_t( b ) + 1] - off[size_t( b )] );
+   }
+   if ( sf.tiles > kSurfaceMaxTiles || surfaceSmem( sf, sizeof( float ) ) > kSurfaceMaxSmem )
+   {
+      sf = SurfaceDev{};
+      return;
+   }
+   lh.faceTiles.upload( tiles );
+   lh.faceTileOff.upload( off );
+   sf.tile    = lh.faceTiles.p;
+   sf.tileOff = lh.faceTileOff.p;
+   sf.list    = lh.colourList.p;
+   sf.m       = s.topo.colours;
+   for ( int c = 0; c < sf.m; ++c )
+      for ( int k = 0; k < 3; ++k )
+         sf.off[c][k] = lh.colourOff[size_t( 4 * c + k )];
+}
 
 void buildStorage( Storage& s, const std::vector< std::array< double, 3 > >& V, const std::vector< std::array< int, 4 > >& T,
                    int maxLevel )
@@ -400,6 +466,7 @@ void buildStorage( Storage& s, const std::vector< std::array< double, 3 > >& V, 
          }
          lh->colourList.upload( flat );
       }
+      buildSurface( s, *lh );
       s.lv.push_back( std::move( lh ) );
    }
    {
