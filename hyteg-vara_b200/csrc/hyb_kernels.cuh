@@ -2640,76 +2640,143 @@ __device__ double blockSum( double v, double* red )
    return s;
 }
 
-__device__ double cgDot( const TopoDev& tp, const LevelDev& lv, const double* a, const double* b, int flag, double* red )
+// The closure points of a thread in the CG's vector loops (t = threadIdx.x, + blockDim.x, ...):
+// bit k of act and own says whether the k-th has a boundary flag in `flag`, and whether its
+// canonical replica is in its cell too. Found once per solve: looking a point's class up in
+// every loop put a chain of three dependent table reads in front of its two values.
+struct CgPoints
+{
+   unsigned long long act, own;
+};
+__device__ __forceinline__ uint8_t cgFlags( const TopoDev& tp, const LevelDev& lv, int cell, int idx, int flag )
+{
+   const int       p  = lv.xyz[idx];
+   const ClassDev& cd = tp.cls[cell * 16 + classMask( lv.N, p & 1023, ( p >> 10 ) & 1023, p >> 20 )];
+   return uint8_t( ( cd.bc & flag ? 1 : 0 ) | ( ( cd.bc & flag ) && cd.owned ? 2 : 0 ) );
+}
+__device__ __forceinline__ CgPoints cgPoints( const TopoDev& tp, const LevelDev& lv, int flag )
+{
+   CgPoints P{ 0, 0 };
+   int      k = 0;
+   for ( int t = threadIdx.x; t < tp.nC * lv.S && k < 64; t += blockDim.x, ++k )
+   {
+      const uint8_t f = cgFlags( tp, lv, t / lv.S, t % lv.S, flag );
+      P.act |= (unsigned long long) ( f & 1 ) << k;
+      P.own |= (unsigned long long) ( f >> 1 ) << k;
+   }
+   return P;
+}
+// f( i ) for every slab index i of the thread's active (OWNED: and owned) points; LISTS as in
+// cgBody
+template < bool LISTS, bool OWNED, typename F >
+__device__ __forceinline__ void cgForEach( const TopoDev& tp, const LevelDev& lv, const CgPoints& P, int flag, F&& f )
+{
+   int k = 0;
+   for ( int t = threadIdx.x; t < tp.nC * lv.S; t += blockDim.x, ++k )
+   {
+      const int  cell = t / lv.S, idx = t % lv.S;
+      const bool on   = LISTS && k < 64 ? ( ( OWNED ? P.own : P.act ) >> k ) & 1
+                                        : ( cgFlags( tp, lv, cell, idx, flag ) & ( OWNED ? 2 : 1 ) ) != 0;
+      if ( on )
+         f( size_t( cell ) * lv.stride + idx );
+   }
+}
+
+template < bool LISTS >
+__device__ double cgDot( const TopoDev& tp, const LevelDev& lv, const CgPoints& P, const double* a, const double* b, int flag,
+                         double* red )
 {
    double v = 0;
-   for ( int t = threadIdx.x; t < tp.nC * lv.S; t += blockDim.x )
-   {
-      const int cell = t / lv.S, idx = t % lv.S;
-      const int p    = lv.xyz[idx];
-      const ClassDev cd = tp.cls[cell * 16 + classMask( lv.N, p & 1023, ( p >> 10 ) & 1023, p >> 20 )];
-      if ( cd.owned && ( cd.bc & flag ) )
-         v += a[size_t( cell ) * lv.stride + idx] * b[size_t( cell ) * lv.stride + idx];
-   }
+   cgForEach< LISTS, true >( tp, lv, P, flag, [&]( size_t i ) { v += a[i] * b[i]; } );
    return blockSum( v, red );
 }
 
 // y = a*x + b*y over flagged points of all replicas
-__device__ void cgAxpby( const TopoDev& tp, const LevelDev& lv, double a, const double* x, double b, double* y, int flag )
+template < bool LISTS >
+__device__ void cgAxpby( const TopoDev& tp, const LevelDev& lv, const CgPoints& P, double a, const double* x, double b,
+                         double* y, int flag )
 {
-   for ( int t = threadIdx.x; t < tp.nC * lv.S; t += blockDim.x )
-   {
-      const int cell = t / lv.S, idx = t % lv.S;
-      const int p    = lv.xyz[idx];
-      if ( !( tp.cls[cell * 16 + classMask( lv.N, p & 1023, ( p >> 10 ) & 1023, p >> 20 )].bc & flag ) )
-         continue;
-      const size_t i = size_t( cell ) * lv.stride + idx;
-      y[i]           = a * x[i] + b * y[i];
-   }
+   cgForEach< LISTS, false >( tp, lv, P, flag, [&]( size_t i ) { y[i] = a * x[i] + b * y[i]; } );
 }
 
-// the whole CG in the calling thread block; red = 32 doubles of shared memory
-template < int VAR, bool BLEND = false >
+constexpr int kCgGroups = 512; // listed lane groups of the CG's operator at most; above it every group runs
+
+// the whole CG in the calling thread block; red = 32 doubles of shared memory. LISTS: the active
+// points and rows are listed first (k_cg: 147 -> 142 ms for a mixed lognormal solve on 384
+// cells, of which the CG runs 16 times); in the program kernels, whose level 0 has a handful of
+// unknowns, the lists cost more than they save (twelve served requests 66 ms, with them 68).
+template < int VAR, bool BLEND = false, bool LISTS = false >
 __device__ void cgBody( const TopoDev& tp, const LevelDev& lv, const OpDev< double >& op, double* x, const double* b,
                         double* r, double* p, double* ap, double tol, int maxIter, int* status, double* red,
                         const RowPass& rp )
 {
    const int flag = 1 | 4 | 8;
-   // the operator through the level's row table when there is one
+   // The operator through the level's row table when there is one. On level 0 most vertices lie
+   // on the boundary: the groups of 32 lanes that hold an active row are listed once, so that
+   // the block's warps share those only (384 cells, FP64: 125 groups, 27 of them active).
+   __shared__ int groups[LISTS ? kCgGroups : 1], nGroups;
+   const int      warp = int( threadIdx.x >> 5 ), lane = int( threadIdx.x & 31 ), warps = int( blockDim.x >> 5 );
+   const int      allGroups = int( ( rp.n + 31 ) / 32 );
+   if ( LISTS && rp.rows )
+   {
+      if ( threadIdx.x == 0 )
+         nGroups = 0;
+      __syncthreads();
+      for ( int g = warp; g < allGroups; g += warps )
+      {
+         const long long gt = (long long) g * 32 + lane;
+         bool            on = false;
+         if ( gt < rp.n )
+         {
+            const int4 A = __ldg( reinterpret_cast< const int4* >( rp.rows + gt ) );
+            on           = A.x >= 0 && ( ( A.z >> 16 ) & flag );
+         }
+         if ( __any_sync( 0xffffffffu, on ) && lane == 0 )
+         {
+            const int s = atomicAdd( &nGroups, 1 );
+            if ( s < kCgGroups )
+               groups[s] = g;
+         }
+      }
+      __syncthreads();
+   }
    auto applyA = [&]( const double* src, double* dst ) {
-      if ( BLEND || rp.rows )
+      if ( !LISTS && ( BLEND || rp.rows ) )
          rowPassBody< double, kRowApply, VAR, BLEND >( rp, op, const_cast< double* >( src ), nullptr, dst, 0.0, flag,
                                                        threadIdx.x, blockDim.x );
+      else if ( BLEND || rp.rows )
+      {
+         const bool listed = nGroups <= kCgGroups;
+         const int  n      = listed ? nGroups : allGroups;
+         for ( int i = warp; i < n; i += warps )
+            rowPassBody< double, kRowApply, VAR, BLEND >( rp, op, const_cast< double* >( src ), nullptr, dst, 0.0, flag,
+                                                          ( listed ? groups[i] : i ) * 32ll + lane, rp.n + 32 );
+      }
       else
          cgApplyAll< VAR >( tp, lv, op, src, dst, flag );
    };
    applyA( x, p );
    __syncthreads();
    // r = b - A x ; p = r
-   for ( int t = threadIdx.x; t < tp.nC * lv.S; t += blockDim.x )
-   {
-      const int cell = t / lv.S, idx = t % lv.S;
-      const int pp   = lv.xyz[idx];
-      if ( !( tp.cls[cell * 16 + classMask( lv.N, pp & 1023, ( pp >> 10 ) & 1023, pp >> 20 )].bc & flag ) )
-         continue;
-      const size_t i = size_t( cell ) * lv.stride + idx;
-      r[i]           = b[i] - p[i];
-      p[i]           = r[i];
-   }
+   const CgPoints pts = LISTS ? cgPoints( tp, lv, flag ) : CgPoints{ 0, 0 };
+   cgForEach< LISTS, false >( tp, lv, pts, flag, [&]( size_t i ) {
+      r[i] = b[i] - p[i];
+      p[i] = r[i];
+   } );
    __syncthreads();
-   double prsold = cgDot( tp, lv, r, r, flag, red );
+   double prsold = cgDot< LISTS >( tp, lv, pts, r, r, flag, red );
    int    it     = 0;
    int    conv   = sqrt( prsold ) < tol ? 1 : 0;
    while ( !conv && it < maxIter )
    {
       applyA( p, ap );
       __syncthreads();
-      const double pAp   = cgDot( tp, lv, p, ap, flag, red );
+      const double pAp   = cgDot< LISTS >( tp, lv, pts, p, ap, flag, red );
       const double alpha = prsold / pAp;
-      cgAxpby( tp, lv, alpha, p, 1.0, x, flag );
-      cgAxpby( tp, lv, -alpha, ap, 1.0, r, flag );
+      cgAxpby< LISTS >( tp, lv, pts, alpha, p, 1.0, x, flag );
+      cgAxpby< LISTS >( tp, lv, pts, -alpha, ap, 1.0, r, flag );
       __syncthreads();
-      const double rsnew = cgDot( tp, lv, r, r, flag, red );
+      const double rsnew = cgDot< LISTS >( tp, lv, pts, r, r, flag, red );
       ++it;
       if ( sqrt( rsnew ) < tol )
       {
@@ -2717,7 +2784,7 @@ __device__ void cgBody( const TopoDev& tp, const LevelDev& lv, const OpDev< doub
          break;
       }
       const double beta = rsnew / prsold;
-      cgAxpby( tp, lv, 1.0, r, beta, p, flag );
+      cgAxpby< LISTS >( tp, lv, pts, 1.0, r, beta, p, flag );
       __syncthreads();
       prsold = rsnew;
    }
@@ -2729,13 +2796,13 @@ __device__ void cgBody( const TopoDev& tp, const LevelDev& lv, const OpDev< doub
 }
 
 template < int VAR, bool BLEND = false >
-__global__ void __launch_bounds__( 256 ) k_cg( TopoDev tp, LevelDev lv, OpDev< double > op, double* x, const double* b,
+__global__ void __launch_bounds__( BLEND ? 256 : 512 ) k_cg( TopoDev tp, LevelDev lv, OpDev< double > op, double* x, const double* b,
                                                 double* r, double* p, double* ap, double tol, int maxIter, int* status,
                                                 RowPass rp )
 {
    HYB_PDL_PROLOGUE();
    __shared__ double red[32];
-   cgBody< VAR, BLEND >( tp, lv, op, x, b, r, p, ap, tol, maxIter, status, red, rp );
+   cgBody< VAR, BLEND, true >( tp, lv, op, x, b, r, p, ap, tol, maxIter, status, red, rp );
 }
 
 // ---------------------------------------------------------------------------

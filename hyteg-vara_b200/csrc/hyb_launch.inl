@@ -505,9 +505,16 @@ void launchSor( const Operator& op, int l, T* u, const T* rhs, T relax, int flag
    auto interfaces = [&]() {
       if ( surfaceSor< T >( op, l, flag ) )
       {
-         HYB_CUDA( launchSurfaceSor< T >( s.td, L.dev, L.surface, od, u, rhs, relax, backwards, stream ) );
-         HYB_CHECK_LAUNCH();
-         return;
+         const cudaError_t e = launchSurfaceSor< T >( s.td, L.dev, L.surface, od, u, rhs, relax, backwards, stream );
+         // a context with fewer SMs than the device (MPS) cannot hold the grid: the colours'
+         // own launches below
+         if ( e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported )
+         {
+            HYB_CUDA( e );
+            HYB_CHECK_LAUNCH();
+            return;
+         }
+         cudaGetLastError();
       }
       for ( int c = 0; c < s.td.m; ++c )
          iface( backwards ? s.td.m - 1 - c : c );
@@ -848,7 +855,7 @@ void launchCg( const Operator& op, int l, double* x, const double* b, CgScratch&
    }
    const RowPass         rp = rowPassAll( rowsIf( s, l ) );
    withVar( op, [&]( auto V ) {
-      pdlLaunch( k_cg< decltype( V )::value >, dim3( 1 ), dim3( 256 ), 0, stream, s.td, s.L( l ).dev, od, x, b,
+      pdlLaunch( k_cg< decltype( V )::value >, dim3( 1 ), dim3( 512 ), 0, stream, s.td, s.L( l ).dev, od, x, b,
                  cs.r->ptr< double >( l ), cs.p->ptr< double >( l ), cs.ap->ptr< double >( l ), tol, maxIter, cs.status.p,
                  rp );
    } );
