@@ -598,10 +598,11 @@ __device__ __forceinline__ void rowPassBody( const RowPass& rp, const OpDev< T >
       T            diag = 0, off = 0, own = 0, bi = 0;
       if ( active )
       {
-         // the point's own value and right-hand side travel with the neighbours
-         if constexpr ( MODE != kRowInvDiag )
+         // the point's own value and right-hand side travel with the neighbours (not in the
+         // blended rows: they are bound by arithmetic, and two more live values spill)
+         if constexpr ( !BLEND && MODE != kRowInvDiag )
             own = u[i];
-         if constexpr ( MODE == kRowSor || MODE == kRowResidual || MODE == kRowJacobi )
+         if constexpr ( !BLEND && ( MODE == kRowSor || MODE == kRowResidual || MODE == kRowJacobi ) )
             bi = b[i];
          const T*       uc    = u + A.x;
          const uint32_t valid = uint32_t( A.z ) & 0xffffu;
@@ -641,6 +642,12 @@ __device__ __forceinline__ void rowPassBody( const RowPass& rp, const OpDev< T >
       off         = groupSum( off, G );
       if ( !active )
          continue;
+      if constexpr ( BLEND )
+      {
+         own = u[i];
+         if constexpr ( MODE == kRowSor || MODE == kRowResidual || MODE == kRowJacobi )
+            bi = b[i];
+      }
       if constexpr ( MODE == kRowSor )
          u[i] = ( T( 1 ) - relax ) * own + relax * ( bi - off ) / diag;
       else if constexpr ( MODE == kRowResidual )

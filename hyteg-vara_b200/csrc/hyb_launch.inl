@@ -386,18 +386,13 @@ static const int kFusedInteriorMaxPoints = [] {
    return e ? std::atoi( e ) : 4096;
 }();
 
-// Whether the interface colours of level l run as one cooperative launch (hyb_surface.cu): from
-// this many surface DoFs on (HYB_SURFACE_MIN_DOFS overrides it). At level 6 on 48 cells (0.25 M)
-// a sweep's six launches take 40 us and the one 61; at level 7 on 48 cells (1 M) 130 against
-// 100, at level 6 on 384 cells (1.8 M, FP32) 165 against 130.
-constexpr long kSurfaceMinDofs = 500000;
+// Whether the interface colours of level l run as one cooperative launch (hyb_surface.cu).
 template < typename T >
 bool surfaceSor( const Operator& op, int l, int flag )
 {
-   static const long  minDofs = envLong( "HYB_SURFACE_MIN_DOFS", kSurfaceMinDofs );
-   const LevelHost&   L       = op.st->L( l );
+   const LevelHost& L = op.st->L( l );
    return varKind( op ) == 0 && !op.blend && flag == ( HYB_INNER | HYB_NEUMANN ) && L.surface.nBlocks > 0 &&
-          L.dev.nBdry >= minDofs && surfaceSmem( L.surface, sizeof( T ) ) <= kSurfaceMaxSmem;
+          surfaceSmem( L.surface, sizeof( T ) ) <= kSurfaceMaxSmem;
 }
 
 template < typename T >

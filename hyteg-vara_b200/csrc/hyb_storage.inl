@@ -109,6 +109,20 @@ struct Storage
 
 inline int stridePad( int s ) { return ( s + 31 ) / 32 * 32; }
 
+// The interface colours of a level run as one cooperative launch (hyb_surface.cu) from this many
+// surface DoFs on (HYB_SURFACE_MIN_DOFS overrides it). At level 6 on 48 cells (0.25 M) a sweep's
+// six launches take 40 us and the one 61; at level 7 on 48 cells (1 M) 130 against 100, at level
+// 6 on 384 cells (1.8 M, FP32) 165 against 130.
+constexpr long kSurfaceMinDofs = 500000;
+inline long    surfaceMinDofs()
+{
+   static const long v = [] {
+      const char* e = std::getenv( "HYB_SURFACE_MIN_DOFS" );
+      return e ? std::atol( e ) : kSurfaceMinDofs;
+   }();
+   return v;
+}
+
 // Deal the inner macro-faces of a level to blocks (SurfaceDev, hyb_surface.cu). A face is cut
 // into `parts` row ranges of about equal size, as few as leave the fullest block the least
 // work: 72 faces on 148 SMs are cut in two, 672 are not cut.
@@ -117,6 +131,8 @@ void buildSurface( const Storage& s, LevelHost& lh )
    const LevelDev& d  = lh.dev;
    SurfaceDev&     sf = lh.surface;
    sf                 = SurfaceDev{};
+   if ( d.nBdry < surfaceMinDofs() )
+      return;
    std::vector< int > faces;
    for ( size_t f = 0; f < s.topo.F.size(); ++f )
       if ( s.topo.fBc[f] == kInner )
@@ -403,6 +419,7 @@ void buildStorage( Storage& s, const std::vector< std::array< double, 3 > >& V, 
             for ( int x = 0; x <= d.N - y - z; ++x )
                xyz[sidx( d.W, x, y, z )] = x | ( y << 10 ) | ( z << 20 );
       std::vector< int32_t > linPos;
+      linPos.reserve( size_t( d.nIntCell ) );
       for ( int z = 1; z <= d.N; ++z )
          for ( int y = 1; y + z <= d.N - 2; ++y )
             for ( int x = 1; x + y + z <= d.N - 1; ++x )
