@@ -846,6 +846,8 @@ __device__ __forceinline__ void applyBody( Blk vb, TopoDev tp, LevelDev lv, OpDe
       T               diag, off, own = 0, b = 0;
       if ( active )
       {
+         // read before the sums: their full-warp shuffles come between every lane's read of the
+         // first replica and the write of it
          const size_t r0 = bdryReplica< T >( tp, lv, p, 0 );
          own             = src[r0];
          if constexpr ( MODE != kReplace )
@@ -871,8 +873,6 @@ __device__ __forceinline__ void applyBody( Blk vb, TopoDev tp, LevelDev lv, OpDe
             bdryWriteGroup( tp, lv, p, tk, cvt, float( v ) );
          continue;
       }
-      // every lane of the group has read dst[r0] before any replica is written
-      __syncwarp( __activemask() );
       bdryWriteGroup( tp, lv, p, tk, dst, v );
    }
 }
@@ -931,6 +931,7 @@ __device__ __forceinline__ void sorIfaceBody( Blk vb, TopoDev tp, LevelDev lv, O
       T               diag, off, own = 0, b = 0;
       if ( active )
       {
+         // (before the sums, as in applyBody)
          const size_t r0 = bdryReplica< T >( tp, lv, p, 0 );
          own             = u[r0];
          b               = rhs[r0];
@@ -939,8 +940,6 @@ __device__ __forceinline__ void sorIfaceBody( Blk vb, TopoDev tp, LevelDev lv, O
       if ( !active )
          continue;
       const T v = ( T( 1 ) - relax ) * own + relax * ( b - off ) / diag;
-      // all lanes of the group read u[r0] before any replica is written
-      __syncwarp( __activemask() );
       bdryWriteGroup( tp, lv, p, tk, u, v );
    }
 }
@@ -2038,17 +2037,21 @@ __device__ __forceinline__ void prolongateBody( Blk vb, TopoDev tp, LevelDev lv,
    const BdryLists bl = fullBdryLists( tp, lv );
    HYB_BDRY_LANES( bl )
    {
-      const LaneTask  tk = laneTask( tp, lv, bl, gt );
-      const BdryPoint p  = decodeBdry( tp, lv, tk.t );
-      if ( !tk.valid || !( primBc( tp, p.kind, p.prim ) & flag ) )
+      const LaneTask  tk     = laneTask( tp, lv, bl, gt );
+      const BdryPoint p      = decodeBdry( tp, lv, tk.t );
+      const bool      active = tk.valid && ( primBc( tp, p.kind, p.prim ) & flag );
+      T               v      = 0;
+      if ( active )
+      {
+         int c, x, y, z;
+         embeddingCoords( embAt( tp, p.kind, p.prim, 0 ), p.kind, lv.N, p.i, p.j, c, x, y, z );
+         v = interpolateFine( coarse + size_t( c ) * strideC, Wc, x, y, z );
+         if ( ADD )
+            v += fine[size_t( c ) * lv.stride + sidx( lv.W, x, y, z )];
+      }
+      __syncwarp(); // every lane of a group has read the old value before a replica is written
+      if ( !active )
          continue;
-      int c, x, y, z;
-      embeddingCoords( embAt( tp, p.kind, p.prim, 0 ), p.kind, lv.N, p.i, p.j, c, x, y, z );
-      T v = interpolateFine( coarse + size_t( c ) * strideC, Wc, x, y, z );
-      if ( ADD )
-         v += fine[size_t( c ) * lv.stride + sidx( lv.W, x, y, z )];
-      // every lane of the group has read the old value before any replica is written
-      __syncwarp( __activemask() );
       bdryWriteGroup( tp, lv, p, tk, fine, v );
    }
 }

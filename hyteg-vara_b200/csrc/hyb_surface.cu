@@ -280,10 +280,15 @@ __global__ void __launch_bounds__( kSurfaceThreads, 1 )
             const LaneTask  tk     = laneTask( tp, lv, bl, gt );
             const BdryPoint p      = decodeBdry( tp, lv, tk.t );
             const bool      active = tk.valid && ( primBc( tp, p.kind, p.prim ) & ( 1 | 4 ) );
-            T               diag = 0, off = 0;
+            T               diag = 0, off = 0, own = 0, b = 0;
             if ( active )
             {
-               const int ne = numEmb( tp, p.kind, p.prim );
+               // read before the sums: their full-warp shuffles come between every lane's read
+               // of the first replica and the write of it
+               const size_t r0 = bdryReplica< T >( tp, lv, p, 0 );
+               own             = __ldcg( u + r0 );
+               b               = rhs[r0];
+               const int ne    = numEmb( tp, p.kind, p.prim );
                for ( int e = tk.sub; e < ne; e += tk.G )
                {
                   int cell, x, y, z;
@@ -295,9 +300,7 @@ __global__ void __launch_bounds__( kSurfaceThreads, 1 )
             off  = groupSum( off, tk.G );
             if ( !active )
                continue;
-            const size_t r0 = bdryReplica< T >( tp, lv, p, 0 );
-            const T      v  = ( T( 1 ) - relax ) * __ldcg( u + r0 ) + relax * ( rhs[r0] - off ) / diag;
-            __syncwarp( __activemask() ); // every lane has read u[r0]
+            const T v = ( T( 1 ) - relax ) * own + relax * ( b - off ) / diag;
             bdryWriteGroup( tp, lv, p, tk, u, v );
          }
       }
