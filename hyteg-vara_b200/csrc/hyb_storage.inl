@@ -177,6 +177,7 @@ void buildSurface( const Storage& s, LevelHost& lh )
       sf = SurfaceDev{};
       return;
    }
+   HYB_CUDA( surfacePrepare() );
    lh.faceTiles.upload( tiles );
    lh.faceTileOff.upload( off );
    sf.tile    = lh.faceTiles.p;

@@ -375,14 +375,17 @@ __global__ void __launch_bounds__( kSurfaceThreads, 1 )
 
 size_t surfaceSmem( const SurfaceDev& sf, int elem ) { return size_t( sf.most ) * ( 2 * elem + 2 ) + 16; }
 
+cudaError_t surfacePrepare()
+{
+   const cudaFuncAttribute a  = cudaFuncAttributeMaxDynamicSharedMemorySize;
+   const cudaError_t       e = cudaFuncSetAttribute( k_surface_sor< float >, a, int( kSurfaceMaxSmem ) );
+   return e != cudaSuccess ? e : cudaFuncSetAttribute( k_surface_sor< double >, a, int( kSurfaceMaxSmem ) );
+}
+
 template < typename T >
 cudaError_t launchSurfaceSor( const TopoDev& tp, const LevelDev& lv, const SurfaceDev& sf, const OpDev< T >& op, T* u,
                               const T* rhs, T relax, bool backwards, cudaStream_t stream )
 {
-   static const cudaError_t attr =
-       cudaFuncSetAttribute( k_surface_sor< T >, cudaFuncAttributeMaxDynamicSharedMemorySize, int( kSurfaceMaxSmem ) );
-   if ( attr != cudaSuccess )
-      return attr;
    cudaLaunchConfig_t  c{};
    cudaLaunchAttribute a{};
    a.id               = cudaLaunchAttributeCooperative;

@@ -34,6 +34,10 @@ constexpr int kSurfaceMaxTiles   = 16; // tiles a block takes at most
 size_t           surfaceSmem( const SurfaceDev& sf, int elem );
 constexpr size_t kSurfaceMaxSmem = 200 * 1024;
 
+// Lets the launch have that much shared memory on the current device. The opt-in is kept per
+// device: every storage that has tiles calls this when it is built.
+cudaError_t surfacePrepare();
+
 // All interface colours of one sweep (in the order 0 .. m-1, backwards: m-1 .. 0), for the
 // DoFs on Inner | Neumann. A cooperative launch.
 template < typename T >
