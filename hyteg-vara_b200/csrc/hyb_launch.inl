@@ -501,9 +501,8 @@ void launchSor( const Operator& op, int l, T* u, const T* rhs, T relax, int flag
       if ( surfaceSor< T >( op, l, flag ) )
       {
          const cudaError_t e = launchSurfaceSor< T >( s.td, L.dev, L.surface, od, u, rhs, relax, backwards, stream );
-         // a context with fewer SMs than the device (MPS) cannot hold the grid: the colours'
-         // own launches below
-         if ( e != cudaErrorCooperativeLaunchTooLarge && e != cudaErrorNotSupported )
+         // a stream whose part of the device cannot hold the grid: the colours' own launches below
+         if ( e != cudaErrorCooperativeLaunchTooLarge )
          {
             HYB_CUDA( e );
             HYB_CHECK_LAUNCH();

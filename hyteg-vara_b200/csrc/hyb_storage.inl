@@ -172,12 +172,14 @@ void buildSurface( const Storage& s, LevelHost& lh )
       sf.most  = std::max( sf.most, ( held + 7 ) / 8 * 8 );
       sf.tiles = std::max( sf.tiles, off[size_t( b ) + 1] - off[size_t( b )] );
    }
-   if ( sf.tiles > kSurfaceMaxTiles || surfaceSmem( sf, sizeof( float ) ) > kSurfaceMaxSmem )
+   bool fits = sf.tiles <= kSurfaceMaxTiles && surfaceSmem( sf, sizeof( float ) ) <= kSurfaceMaxSmem;
+   if ( fits )
+      HYB_CUDA( surfacePrepare( sf, &fits ) );
+   if ( !fits )
    {
       sf = SurfaceDev{};
       return;
    }
-   HYB_CUDA( surfacePrepare() );
    lh.faceTiles.upload( tiles );
    lh.faceTileOff.upload( off );
    sf.tile    = lh.faceTiles.p;

@@ -3,8 +3,10 @@
 #include "hyb_surface.hpp"
 
 #include <algorithm>
+#include <type_traits>
 
 #include <cooperative_groups.h>
+#include <cuda.h>
 
 #include "hyb_surface_dofs.cuh"
 
@@ -375,17 +377,86 @@ __global__ void __launch_bounds__( kSurfaceThreads, 1 )
 
 size_t surfaceSmem( const SurfaceDev& sf, int elem ) { return size_t( sf.most ) * ( 2 * elem + 2 ) + 16; }
 
-cudaError_t surfacePrepare()
+namespace {
+// one block of every SM of the current device has room for the launch in T, and the opt-in to its
+// shared memory is set
+template < typename T >
+cudaError_t prepareFor( const SurfaceDev& sf, int sms, bool* fits )
 {
-   const cudaFuncAttribute a  = cudaFuncAttributeMaxDynamicSharedMemorySize;
-   const cudaError_t       e = cudaFuncSetAttribute( k_surface_sor< float >, a, int( kSurfaceMaxSmem ) );
-   return e != cudaSuccess ? e : cudaFuncSetAttribute( k_surface_sor< double >, a, int( kSurfaceMaxSmem ) );
+   const cudaError_t e =
+       cudaFuncSetAttribute( k_surface_sor< T >, cudaFuncAttributeMaxDynamicSharedMemorySize, int( kSurfaceMaxSmem ) );
+   if ( e != cudaSuccess || surfaceSmem( sf, sizeof( T ) ) > kSurfaceMaxSmem )
+      return e; // (the value types are asked for one by one: surfaceSor)
+   int               perSM = 0;
+   const cudaError_t o     = cudaOccupancyMaxActiveBlocksPerMultiprocessor( &perSM, k_surface_sor< T >, kSurfaceThreads,
+                                                                        surfaceSmem( sf, sizeof( T ) ) );
+   *fits                   = *fits && perSM * sms >= sf.nBlocks;
+   return o;
+}
+
+// SMs of the context (or its partition) that the stream's kernels run on; 0 where the driver
+// does not say
+int streamSMs( cudaStream_t stream )
+{
+   struct Driver
+   {
+      CUresult ( *streamCtx )( CUstream, CUcontext*, CUgreenCtx* )                      = nullptr;
+      CUresult ( *ctxResource )( CUcontext, CUdevResource*, CUdevResourceType )         = nullptr;
+      CUresult ( *greenCtxResource )( CUgreenCtx, CUdevResource*, CUdevResourceType ) = nullptr;
+   };
+   static const Driver d = [] {
+      Driver r;
+      auto   get = []( const char* name, auto& f ) {
+         void*                           p = nullptr;
+         cudaDriverEntryPointQueryResult q;
+         if ( cudaGetDriverEntryPointByVersion( name, &p, 12050, cudaEnableDefault, &q ) == cudaSuccess &&
+              q == cudaDriverEntryPointSuccess )
+            f = reinterpret_cast< std::decay_t< decltype( f ) > >( p );
+         else
+            cudaGetLastError();
+      };
+      get( "cuStreamGetCtx", r.streamCtx ); // from 12.5 on: with the stream's green context
+      get( "cuCtxGetDevResource", r.ctxResource );
+      get( "cuGreenCtxGetDevResource", r.greenCtxResource );
+      return r;
+   }();
+   CUcontext     ctx   = nullptr;
+   CUgreenCtx    green = nullptr;
+   CUdevResource sm{};
+   if ( !d.streamCtx || !d.ctxResource || !d.greenCtxResource || d.streamCtx( stream, &ctx, &green ) != CUDA_SUCCESS )
+      return 0;
+   const CUresult r = green ? d.greenCtxResource( green, &sm, CU_DEV_RESOURCE_TYPE_SM )
+                            : d.ctxResource( ctx, &sm, CU_DEV_RESOURCE_TYPE_SM );
+   return r == CUDA_SUCCESS ? int( sm.sm.smCount ) : 0;
+}
+} // namespace
+
+cudaError_t surfacePrepare( const SurfaceDev& sf, bool* fits )
+{
+   int         dev = 0, coop = 0, mps = 0, sms = 0;
+   cudaError_t e   = cudaGetDevice( &dev );
+   if ( e == cudaSuccess )
+      e = cudaDeviceGetAttribute( &coop, cudaDevAttrCooperativeLaunch, dev );
+   if ( e == cudaSuccess )
+      e = cudaDeviceGetAttribute( &mps, cudaDevAttrMpsEnabled, dev );
+   if ( e == cudaSuccess )
+      e = cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev );
+   *fits = coop && !mps;
+   if ( e == cudaSuccess )
+      e = prepareFor< float >( sf, sms, fits );
+   if ( e == cudaSuccess )
+      e = prepareFor< double >( sf, sms, fits );
+   return e;
 }
 
 template < typename T >
 cudaError_t launchSurfaceSor( const TopoDev& tp, const LevelDev& lv, const SurfaceDev& sf, const OpDev< T >& op, T* u,
                               const T* rhs, T relax, bool backwards, cudaStream_t stream )
 {
+   // A captured launch is refused only when its graph is instantiated or run, so the grid is
+   // held against the stream's SMs here (one resident block each) and not left to the launch.
+   if ( streamSMs( stream ) < sf.nBlocks )
+      return cudaErrorCooperativeLaunchTooLarge;
    cudaLaunchConfig_t  c{};
    cudaLaunchAttribute a{};
    a.id               = cudaLaunchAttributeCooperative;

@@ -34,12 +34,16 @@ constexpr int kSurfaceMaxTiles   = 16; // tiles a block takes at most
 size_t           surfaceSmem( const SurfaceDev& sf, int elem );
 constexpr size_t kSurfaceMaxSmem = 200 * 1024;
 
-// Lets the launch have that much shared memory on the current device. The opt-in is kept per
-// device: every storage that has tiles calls this when it is built.
-cudaError_t surfacePrepare();
+// Sets up the launch on the current device (the opt-in to its shared memory is kept per device:
+// every storage that has tiles calls this when it is built) and tells whether the device can run
+// it: with room for the whole grid, and not under MPS, where a cooperative launch is not allowed
+// in the body of a graph's loop, as the device-iterated solves have it.
+cudaError_t surfacePrepare( const SurfaceDev& sf, bool* fits );
 
 // All interface colours of one sweep (in the order 0 .. m-1, backwards: m-1 .. 0), for the
-// DoFs on Inner | Neumann. A cooperative launch.
+// DoFs on Inner | Neumann. A cooperative launch; cudaErrorCooperativeLaunchTooLarge, captured or
+// not and with nothing launched, when the stream's SMs (a green context's part of the device)
+// cannot hold the grid.
 template < typename T >
 cudaError_t launchSurfaceSor( const TopoDev& tp, const LevelDev& lv, const SurfaceDev& sf, const OpDev< T >& op, T* u,
                               const T* rhs, T relax, bool backwards, cudaStream_t stream );

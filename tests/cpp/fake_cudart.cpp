@@ -2,12 +2,33 @@
 // here: a kernel's shared-memory opt-in is kept per device, as the runtime keeps it.
 #include "fake_cudart.hpp"
 
+#include <cstring>
 #include <map>
+
+#include <cuda.h>
 
 FakeCuda fake;
 
 namespace {
 std::map< const void*, int > optIn[2]; // by device: kernel -> bytes of dynamic shared memory allowed
+int                          a_green;
+
+CUresult streamCtx( CUstream, CUcontext* c, CUgreenCtx* g )
+{
+   *c = nullptr;
+   *g = fake.greenSMs ? reinterpret_cast< CUgreenCtx >( &a_green ) : nullptr;
+   return CUDA_SUCCESS;
+}
+CUresult ctxResource( CUcontext, CUdevResource* r, CUdevResourceType )
+{
+   r->sm.smCount = unsigned( fake.ctxSMs );
+   return CUDA_SUCCESS;
+}
+CUresult greenResource( CUgreenCtx, CUdevResource* r, CUdevResourceType )
+{
+   r->sm.smCount = unsigned( fake.greenSMs );
+   return CUDA_SUCCESS;
+}
 }
 
 extern "C" {
@@ -30,6 +51,36 @@ cudaError_t cudaFuncSetAttribute( const void* f, cudaFuncAttribute a, int v )
 {
    if ( a == cudaFuncAttributeMaxDynamicSharedMemorySize )
       optIn[fake.device][f] = v;
+   return cudaSuccess;
+}
+cudaError_t cudaGetDevice( int* d )
+{
+   *d = fake.device;
+   return cudaSuccess;
+}
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+cudaError_t cudaDeviceGetAttribute( int* v, cudaDeviceAttr a, int )
+{
+   *v = a == cudaDevAttrCooperativeLaunch ? fake.cooperative : a == cudaDevAttrMpsEnabled ? fake.mps : fake.sms;
+   return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessorWithFlags( int* n, const void*, int, size_t, unsigned )
+{
+   *n = fake.perSM;
+   return cudaSuccess;
+}
+cudaError_t cudaOccupancyMaxActiveBlocksPerMultiprocessor( int* n, const void*, int, size_t )
+{
+   *n = fake.perSM;
+   return cudaSuccess;
+}
+cudaError_t cudaGetDriverEntryPointByVersion( const char* name, void** f, unsigned, unsigned long long,
+                                              cudaDriverEntryPointQueryResult* q )
+{
+   *f = !std::strcmp( name, "cuStreamGetCtx" )        ? reinterpret_cast< void* >( streamCtx )
+        : !std::strcmp( name, "cuCtxGetDevResource" ) ? reinterpret_cast< void* >( ctxResource )
+                                                      : reinterpret_cast< void* >( greenResource );
+   *q = fake.noDriver ? cudaDriverEntryPointSymbolNotFound : cudaDriverEntryPointSuccess;
    return cudaSuccess;
 }
 cudaError_t cudaLaunchKernelExC( const cudaLaunchConfig_t* c, const void* f, void** )

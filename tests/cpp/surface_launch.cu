@@ -25,15 +25,22 @@ cudaError_t launch( const SurfaceDev& sf )
    return launchSurfaceSor< T >( tp, lv, sf, op, nullptr, nullptr, T( 1 ), false, nullptr );
 }
 
-// two devices of one process, each with its own storage: both launch above 48 KB
-int devices()
+SurfaceDev tiles()
 {
    SurfaceDev sf{};
    sf.nBlocks = 148;
    sf.most    = 8000; // 144 KB in FP64
+   return sf;
+}
+
+// two devices of one process, each with its own storage: both launch above 48 KB
+int devices()
+{
+   const SurfaceDev sf = tiles();
    for ( fake.device = 0; fake.device < 2; ++fake.device )
    {
-      CHECK( surfacePrepare() == cudaSuccess );
+      bool fits = false;
+      CHECK( surfacePrepare( sf, &fits ) == cudaSuccess && fits );
       CHECK( launch< double >( sf ) == cudaSuccess );
       CHECK( launch< float >( sf ) == cudaSuccess );
    }
@@ -41,9 +48,62 @@ int devices()
    return 0;
 }
 
+// whether a storage keeps its tiles: decided when it is built, so that no solve that is captured
+// into a graph holds a launch the device cannot run
+int fits()
+{
+   auto kept = []( auto&& change ) {
+      fake = FakeCuda{};
+      change();
+      bool f = false;
+      return surfacePrepare( tiles(), &f ) == cudaSuccess && f;
+   };
+   CHECK( kept( [] {} ) );
+   CHECK( !kept( [] { fake.mps = 1; } ) );
+   CHECK( !kept( [] { fake.cooperative = 0; } ) );
+   CHECK( !kept( [] { fake.perSM = 0; } ) );
+   CHECK( !kept( [] { fake.sms = 147; } ) );
+   CHECK( kept( [] { fake.sms = 74, fake.perSM = 2; } ) );
+   return 0;
+}
+
+// a stream on a part of the device: refused before anything is launched or captured
+int stream()
+{
+   const SurfaceDev sf = tiles();
+   auto             launched = [&]( auto&& change ) {
+      fake     = FakeCuda{};
+      bool   f = false;
+      change();
+      return surfacePrepare( sf, &f ) == cudaSuccess && launch< float >( sf ) == cudaSuccess && fake.launches == 1;
+   };
+   CHECK( launched( [] {} ) );
+   CHECK( !launched( [] { fake.greenSMs = 64; } ) );
+   CHECK( launch< float >( sf ) == cudaErrorCooperativeLaunchTooLarge && fake.launches == 0 );
+   CHECK( launched( [] { fake.greenSMs = 148; } ) );
+   CHECK( !launched( [] { fake.ctxSMs = 100; } ) );
+   return 0;
+}
+
+// a driver that does not say how many SMs a stream has
+int silent()
+{
+   fake.noDriver = true;
+   bool f        = false;
+   CHECK( surfacePrepare( tiles(), &f ) == cudaSuccess );
+   CHECK( launch< double >( tiles() ) == cudaErrorCooperativeLaunchTooLarge && fake.launches == 0 );
+   return 0;
+}
+
 int main( int, char** argv )
 {
-   if ( !std::strcmp( argv[1], "devices" ) )
-      return devices();
+   struct
+   {
+      const char* name;
+      int ( *f )();
+   } const checks[] = { { "devices", devices }, { "fits", fits }, { "stream", stream }, { "silent", silent } };
+   for ( const auto& c : checks )
+      if ( !std::strcmp( argv[1], c.name ) )
+         return c.f();
    return 2;
 }
