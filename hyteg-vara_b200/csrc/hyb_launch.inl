@@ -535,18 +535,19 @@ template < typename T >
 void sorRefPrepare( Storage& s, int l )
 {
    ensureLex( s, l );
-   static const bool attrs = [] {
-      const int mx = int( kSorRefMaxSmem );
-      const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
-      HYB_CUDA( cudaFuncSetAttribute( k_sorref_cells_wave< T, 0 >, a, mx ) );
-      HYB_CUDA( cudaFuncSetAttribute( k_sorref_cells_wave< T, 1 >, a, mx ) );
-      HYB_CUDA( cudaFuncSetAttribute( k_sorref_faces_stage< T, 0 >, a, mx ) );
-      HYB_CUDA( cudaFuncSetAttribute( k_sorref_faces_stage< T, 1 >, a, mx ) );
-      HYB_CUDA( cudaFuncSetAttribute( k_sorref_cells_stage< T, 0 >, a, mx ) );
-      HYB_CUDA( cudaFuncSetAttribute( k_sorref_cells_stage< T, 1 >, a, mx ) );
-      return true;
-   }();
-   (void) attrs;
+   // (kept with the storage, as the opt-in holds for one device)
+   bool& set = s.sorRefOptIn[sizeof( T ) == 8];
+   if ( set )
+      return;
+   const int mx = int( kSorRefMaxSmem );
+   const cudaFuncAttribute a = cudaFuncAttributeMaxDynamicSharedMemorySize;
+   HYB_CUDA( cudaFuncSetAttribute( k_sorref_cells_wave< T, 0 >, a, mx ) );
+   HYB_CUDA( cudaFuncSetAttribute( k_sorref_cells_wave< T, 1 >, a, mx ) );
+   HYB_CUDA( cudaFuncSetAttribute( k_sorref_faces_stage< T, 0 >, a, mx ) );
+   HYB_CUDA( cudaFuncSetAttribute( k_sorref_faces_stage< T, 1 >, a, mx ) );
+   HYB_CUDA( cudaFuncSetAttribute( k_sorref_cells_stage< T, 0 >, a, mx ) );
+   HYB_CUDA( cudaFuncSetAttribute( k_sorref_cells_stage< T, 1 >, a, mx ) );
+   set = true;
 }
 
 // Reference-order SOR: the staged lexicographic sweep of the reference's smooth_sor /

@@ -98,6 +98,8 @@ struct Storage
       return reinterpret_cast< T* >( sorCoef.p );
    }
 
+   bool sorRefOptIn[2] = {}; // FP32, FP64: the reference-order SOR's shared memory is opted in (sorRefPrepare)
+
    ~Storage()
    {
       if ( hostScalar )

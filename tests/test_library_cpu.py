@@ -331,3 +331,16 @@ def test_chebyshev_coefficients(lib, oracle_mod, order):
     np.testing.assert_allclose(r, Tk((th - lam) / de) / Tk(th / de), atol=1e-12)
     with pytest.raises(H.HybError):
         H.chebyshev_coefficients(6, lo, hi)
+
+
+def test_kernel_attributes_are_not_set_once_per_process():
+    # cudaFuncSetAttribute holds for the current device: behind a function-local static a second
+    # device of the process would never get it
+    csrc = os.path.join(PKG, "csrc")
+    found = 0
+    for f in sorted(os.listdir(csrc)):
+        text = re.sub(r"//[^\n]*", "", open(os.path.join(csrc, f)).read())
+        found += text.count("cudaFuncSetAttribute")
+        for m in re.finditer(r"\bstatic\s+const\s+\w+\s+\w+\s*=\s*(\[\]\s*\{.*?\}\(\)|[^;]*);", text, re.S):
+            assert "cudaFuncSetAttribute" not in m.group(0), (f, m.group(0)[:120])
+    assert found
