@@ -294,7 +294,8 @@ void buildStorage( Storage& s, const std::vector< std::array< double, 3 > >& V, 
       d.nIntFace   = d.N >= 3 ? ( d.N - 1 ) * ( d.N - 2 ) / 2 : 0;
       d.nIntCell   = d.N >= 4 ? tetSize( d.N - 3 ) : 0;
       d.nBdry      = nV + nE * ( d.N - 1 ) + nF * d.nIntFace;
-      std::vector< int32_t >                seg, xyz( d.S ), blk, blkXYZ, pts, quads, rowYZ;
+      std::vector< int32_t >                seg, blk, blkXYZ, pts, quads, rowYZ;
+      std::vector< int32_t >                xyz( size_t( d.S ) + size_t( d.nIntCell ) ); // [S] LevelDev::xyz, then linPos
       std::vector< std::vector< int32_t > > ptsC( kInteriorColours );
       for ( int z = 1; z <= d.N; ++z )
          for ( int y = 1; y <= d.N - z; ++y )
@@ -314,10 +315,14 @@ void buildStorage( Storage& s, const std::vector< std::array< double, 3 > >& V, 
       // positions whose neighbour offsets agree (checked, not assumed from the layout)
       {
          std::vector< std::array< int, 2 > > order; // (position, packed x | y << 10 | z << 20)
+         order.reserve( size_t( d.nIntCell ) );
          for ( int z = 1; z <= d.N; ++z )
             for ( int y = 1; y + z <= d.N - 2; ++y )
                for ( int x = 1; x + y + z <= d.N - 1; ++x )
                   order.push_back( { sidx( d.W, x, y, z ), x | ( y << 10 ) | ( z << 20 ) } );
+         require( int( order.size() ) == d.nIntCell, "interior point count" );
+         for ( size_t i = 0; i < order.size(); ++i ) // still in tet-linear order
+            xyz[size_t( d.S ) + i] = order[i][0];
          std::sort( order.begin(), order.end() );
          int prevPos = -2, start = 0, prevXYZ = -1;
          int prevD[15] = {};
@@ -423,15 +428,7 @@ void buildStorage( Storage& s, const std::vector< std::array< double, 3 > >& V, 
          for ( int y = 0; y <= d.N - z; ++y )
             for ( int x = 0; x <= d.N - y - z; ++x )
                xyz[sidx( d.W, x, y, z )] = x | ( y << 10 ) | ( z << 20 );
-      std::vector< int32_t > linPos;
-      linPos.reserve( size_t( d.nIntCell ) );
-      for ( int z = 1; z <= d.N; ++z )
-         for ( int y = 1; y + z <= d.N - 2; ++y )
-            for ( int x = 1; x + y + z <= d.N - 1; ++x )
-               linPos.push_back( sidx( d.W, x, y, z ) );
-      require( int( linPos.size() ) == d.nIntCell, "interior point count" );
       lh->seg.upload( seg );
-      xyz.insert( xyz.end(), linPos.begin(), linPos.end() ); // one allocation
       lh->xyz.upload( xyz );
       d.nSeg = int( seg.size() );
       d.seg  = lh->seg.p;
