@@ -792,7 +792,7 @@ __device__ __forceinline__ void applyBody( Blk vb, TopoDev tp, LevelDev lv, OpDe
    {
       constexpr int K       = interiorBatch< T, VAR >();
       const int     nChunks = ( lv.nPts + 32 * K - 1 ) / ( 32 * K );
-      // strips as in sorInteriorBody: the cell's weights serve several batches of a warp
+      // strips as in sorInteriorBody; the nodal coefficient's weights serve several batches of a warp
       const int            strip = max( 1, min( kInteriorStrip, tp.nC * nChunks / ( nCellBlocks * int( blockDim.x >> 5 ) ) ) );
       InteriorOp< T, VAR > io;
       int                  loaded = -1;
@@ -801,7 +801,7 @@ __device__ __forceinline__ void applyBody( Blk vb, TopoDev tp, LevelDev lv, OpDe
          const int     cell = it_ / nChunks;
          PointBatch< K > pb;
          pb.load( lv.pts, lv.blk, lv.nPts, ( it_ - cell * nChunks ) * 32 * K + int( threadIdx.x & 31 ) );
-         if ( cell != loaded )
+         if ( VAR != 1 || cell != loaded )
             io.load( op, cell );
          loaded = cell;
          const size_t co = size_t( cell ) * lv.stride;
@@ -968,6 +968,9 @@ __device__ __forceinline__ void sorInteriorBody( Blk vb, TopoDev tp, LevelDev lv
    const int      nChunks = ( nPts + 32 * K - 1 ) / ( 32 * K );
    // strips only while every warp of the grid still gets at least one strip
    const int strip = max( 1, min( kInteriorStrip, tp.nC * nChunks / ( nCellBlocks * int( blockDim.x >> 5 ) ) ) );
+   // nodal coefficient: the cell's edge weights stay over the batches of a strip. The other
+   // operators load theirs for every batch: held across the loop they cost registers (FP64 154
+   // of them against 124, quadrature points 184 against 80) and resident blocks
    InteriorOp< T, VAR > io;
    int                  loaded = -1;
    HYB_CELL_LOOP_STRIP( nChunks, strip )
@@ -976,7 +979,7 @@ __device__ __forceinline__ void sorInteriorBody( Blk vb, TopoDev tp, LevelDev lv
       const int       cell = item / nChunks;
       PointBatch< K > pb;
       pb.load( pts, lv.blk, nPts, ( item - cell * nChunks ) * 32 * K + int( threadIdx.x & 31 ) );
-      if ( cell != loaded )
+      if ( VAR != 1 || cell != loaded )
          io.load( op, cell );
       loaded = cell;
       T*       uc = u + size_t( cell ) * lv.stride;
@@ -1005,9 +1008,9 @@ __device__ __forceinline__ void sorInteriorBody( Blk vb, TopoDev tp, LevelDev lv
 }
 
 // (nodal coefficient: registers for four resident blocks in FP64 and six in FP32 without spills
-// to speak of)
+// to speak of; the others are left to the compiler, which takes up to 184 when asked for one block)
 template < typename T, int VAR >
-__global__ void __launch_bounds__( 128, VAR == 1 ? ( sizeof( T ) == 8 ? 4 : 6 ) : 1 ) k_sor_interior( TopoDev tp, LevelDev lv, OpDev< T > op, T* __restrict__ u,
+__global__ void __launch_bounds__( 128, VAR == 1 ? ( sizeof( T ) == 8 ? 4 : 6 ) : 0 ) k_sor_interior( TopoDev tp, LevelDev lv, OpDev< T > op, T* __restrict__ u,
                                                          const T* __restrict__ rhs, T relax, int colour, int begin,
                                                          int nPts, int nCellBlocks )
 {
