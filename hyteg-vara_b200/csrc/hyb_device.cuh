@@ -429,10 +429,12 @@ __device__ __forceinline__ void rowConstant( const T* st, uint32_t valid, T& dia
    }
 }
 
-// variable coefficient: the offsets `valid` and micro-tets validT around the point; at(q) is the slab position of
-// offset q. The weights of the 14 edges are collected over the tets (three per tet), the
+// variable coefficient: the offsets `valid` and micro-tets validT around the point; at(q) is the
+// slab position of offset q. The weights of the 14 edges are collected over the tets (three per tet), the
 // off-diagonal sum takes one product per edge, and the diagonal is minus the sum of the
-// weights (the element matrices have zero row sums and are symmetric: one entry per pair).
+// weights (the element matrices have zero row sums and are symmetric: one entry per pair). Only
+// the factors of the valid micro-tets are read at quadrature points (half of the 24 on a face): an
+// FP32 residual at level 6 on 384 cells takes 639 us, with all 24 read 836.
 template < typename T, int VAR, typename Val, typename At >
 __device__ __forceinline__ void rowVariable( const OpDev< T >& op, int cell, uint32_t valid, uint32_t validT, T& diag,
                                              T& off, Val&& val, At&& at )
@@ -454,12 +456,12 @@ __device__ __forceinline__ void rowVariable( const OpDev< T >& op, int cell, uin
    for ( int i = 0; i < 24; ++i )
    {
       const IncidentTet it = incidentTet( i );
+      const bool        in = validT & ( 1u << i );
       T                 ks;
       if constexpr ( VAR == 2 )
-         ks = op.kq[( size_t( cell ) * 6 + it.t ) * op.stride + at( it.q[0] )];
+         ks = in ? op.kq[( size_t( cell ) * 6 + it.t ) * op.stride + at( it.q[0] )] : T( 0 );
       else
-         ks = kq[it.q[0]] + kq[it.q[1]] + kq[it.q[2]] + kq[it.q[3]];
-      ks = ( validT & ( 1u << i ) ) ? ks : T( 0 );
+         ks = in ? kq[it.q[0]] + kq[it.q[1]] + kq[it.q[2]] + kq[it.q[3]] : T( 0 );
 #pragma unroll
       for ( int j = 0; j < 4; ++j )
          if ( j != it.k )
