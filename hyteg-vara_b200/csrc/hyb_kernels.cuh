@@ -843,27 +843,24 @@ __device__ __forceinline__ void applyBody( Blk vb, TopoDev tp, LevelDev lv, OpDe
       const LaneTask  tk     = laneTask( tp, lv, bl, gt );
       const BdryPoint p      = decodeBdry( tp, lv, tk.t );
       const bool      active = tk.valid && ( primBc( tp, p.kind, p.prim ) & flag );
-      T               diag, off, own = 0, b = 0;
+      T               diag, off, v = 0;
+      bdryRowGroup< T, VAR, kRowBranch >( tp, lv, op, src, p, tk, active, diag, off );
+      // The point's own value is read after the sums, as held through them it spills: FP64 at level 7
+      // on 48 cells 199 us an apply against 195, a residual 218 against 214.
       if ( active )
       {
-         // read before the sums: their full-warp shuffles come between every lane's read of the
-         // first replica and the write of it
          const size_t r0 = bdryReplica< T >( tp, lv, p, 0 );
-         own             = src[r0];
-         if constexpr ( MODE != kReplace )
-            b = MODE == kAdd ? dst[r0] : rhs[r0];
+         const T      ax = diag * src[r0] + off;
+         if constexpr ( MODE == kReplace )
+            v = ax;
+         else if constexpr ( MODE == kAdd )
+            v = dst[r0] + ax;
+         else
+            v = rhs[r0] - ax;
       }
-      bdryRowGroup< T, VAR, kRowBranch >( tp, lv, op, src, p, tk, active, diag, off );
+      __syncwarp(); // every lane of a group has read dst[r0] or rhs[r0] before a replica is written
       if ( !active )
          continue;
-      const T ax = diag * own + off;
-      T       v;
-      if constexpr ( MODE == kReplace )
-         v = ax;
-      else if constexpr ( MODE == kAdd )
-         v = b + ax;
-      else
-         v = b - ax;
       if constexpr ( MODE == kResidualNorm )
       {
          // the first embedding's lane counts the DoF once; every replica gets float(r)
@@ -931,7 +928,8 @@ __device__ __forceinline__ void sorIfaceBody( Blk vb, TopoDev tp, LevelDev lv, O
       T               diag, off, own = 0, b = 0;
       if ( active )
       {
-         // (before the sums, as in applyBody)
+         // read before the sums: their full-warp shuffles come between every lane's read of the
+         // first replica and the write of it
          const size_t r0 = bdryReplica< T >( tp, lv, p, 0 );
          own             = u[r0];
          b               = rhs[r0];
