@@ -13,7 +13,10 @@ void launchDofs( const Storage& s, int l, T* slab, T* dofs, cudaStream_t stream 
 {
    const auto& L    = s.L( l );
    const int   nInt = ( L.dev.nIntCell + kVecBlock - 1 ) / kVecBlock;
-   const int   nSrf = int( ( L.dev.nBdry + long( kVecThreads ) * s.td.nC - 1 ) / ( long( kVecThreads ) * s.td.nC ) );
+   // threads for the surface DoFs: one each, writing slabs a lane group for vertices and edges
+   const int  nE    = s.td.nE * ( L.dev.N - 1 );
+   const long lanes = TO ? L.dev.nBdry : bdryLaneCount( s.td.nV, nE, 0 ) + ( L.dev.nBdry - s.td.nV - nE );
+   const int  nSrf  = int( ( lanes + long( kVecThreads ) * s.td.nC - 1 ) / ( long( kVecThreads ) * s.td.nC ) );
    pdlLaunch( k_dofs< T, TO >, dim3( nInt + nSrf, s.td.nC ), dim3( kVecThreads ), 0, stream, s.td, L.dev, nInt, slab, dofs );
    HYB_CHECK_LAUNCH();
 }

@@ -2,10 +2,10 @@
 compute it together read one replica and write all of them. The copies have to agree
 afterwards: an operator application reads every cell's own copies, a download only the first,
 so A x on the GPU has to match the oracle's A x of the downloaded x (1e-12 of its largest
-entry in FP64, the bound of the apply's parity tests). Under-relaxed sweeps and the additive
-prolongation, whose results depend on the old value, through each route of the interface
-passes (chosen by environment variables, in a child process): the row tables, a launch per
-colour without tables, one launch for all colours."""
+entry in FP64, the bound of the apply's parity tests). After uploads, and after under-relaxed
+sweeps and the additive prolongation, whose results depend on the old value, through each
+route of the interface passes (chosen by environment variables, in a child process): the row
+tables, a launch per colour without tables, one launch for all colours."""
 import os
 import re
 import subprocess
@@ -45,6 +45,7 @@ def check(mesh, level):
         err = np.abs(y.get(level) - ref).max() / np.abs(ref).max()
         assert err <= 1e-12, (what, err)
 
+    copies_agree("upload")
     for what, step in (("forward", A.smooth_sor), ("backward", A.smooth_sor_backwards)):
         for relax in (0.8, 1.3):
             step(x, b, relax, level, flag)
