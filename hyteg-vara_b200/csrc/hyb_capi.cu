@@ -365,12 +365,11 @@ int hyb_function_interpolate_const( hyb_function* fh, int level, double value, i
    if ( value == 0.0 && flag == HYB_ALL )
       HYB_CUDA( cudaMemsetAsync( f->at( level ), 0, f->levelBytes( level ), S( stream ) ) );
    else if ( f->dtype == HYB_F64 )
-      k_fill< double ><<< dim3( L.vecBlocks, f->st->td.nC ), kVecThreads, 0, S( stream ) >>>( f->st->td, L.dev,
-                                                                                      f->ptr< double >( level ), value, flag );
+      pdlLaunch( k_fill< double >, dim3( L.vecBlocks, f->st->td.nC ), dim3( kVecThreads ), 0, S( stream ), f->st->td, L.dev,
+                 f->ptr< double >( level ), value, flag );
    else
-      k_fill< float ><<< dim3( L.vecBlocks, f->st->td.nC ), kVecThreads, 0, S( stream ) >>>( f->st->td, L.dev,
-                                                                                     f->ptr< float >( level ), float( value ),
-                                                                                     flag );
+      pdlLaunch( k_fill< float >, dim3( L.vecBlocks, f->st->td.nC ), dim3( kVecThreads ), 0, S( stream ), f->st->td, L.dev,
+                 f->ptr< float >( level ), float( value ), flag );
    HYB_CHECK_LAUNCH();
    HYB_API_END
 }
@@ -385,11 +384,11 @@ int hyb_function_fill_uniform_random( hyb_function* fh, int level, uint64_t seed
    const Storage& st = *f->st;
    const auto&    L  = st.L( level );
    if ( f->dtype == HYB_F64 )
-      k_fill_uniform_hash< double ><<< dim3( L.slabBlocks, st.td.nC ), 256, 0, S( stream ) >>>(
-          st.td, L.dev, st.cellCoords.p, st.cellOrder.p, f->ptr< double >( level ), seed, lattice );
+      pdlLaunch( k_fill_uniform_hash< double >, dim3( L.slabBlocks, st.td.nC ), dim3( 256 ), 0, S( stream ), st.td, L.dev,
+                 st.cellCoords.p, st.cellOrder.p, f->ptr< double >( level ), seed, lattice );
    else
-      k_fill_uniform_hash< float ><<< dim3( L.slabBlocks, st.td.nC ), 256, 0, S( stream ) >>>(
-          st.td, L.dev, st.cellCoords.p, st.cellOrder.p, f->ptr< float >( level ), seed, lattice );
+      pdlLaunch( k_fill_uniform_hash< float >, dim3( L.slabBlocks, st.td.nC ), dim3( 256 ), 0, S( stream ), st.td, L.dev,
+                 st.cellCoords.p, st.cellOrder.p, f->ptr< float >( level ), seed, lattice );
    HYB_CHECK_LAUNCH();
    HYB_API_END
 }
