@@ -68,14 +68,14 @@ def check_small_stream():
     orc.sor_colored(ref, b, level, labels, m, relax=0.9, flag=1 | 4)
     for stream, captured, launches in ((None, False, 2), (small, False, m + 1), (small, True, m + 1)):
         x.set(x0, level)
-        ok(rt.cudaDeviceSynchronize() + (None,))
+        ok(rt.cudaStreamSynchronize(0) + (None,))  # the small stream does not wait for the default one
         if captured:
             ok(rt.cudaStreamBeginCapture(stream, rt.cudaStreamCaptureMode.cudaStreamCaptureModeThreadLocal) + (None,))
         assert sweep(stream) == launches
         if captured:
             run = ok(rt.cudaGraphInstantiate(ok(rt.cudaStreamEndCapture(stream)), 0))
             ok(rt.cudaGraphLaunch(run, stream) + (None,))
-        ok(rt.cudaDeviceSynchronize() + (None,))
+        ok(rt.cudaStreamSynchronize(stream or 0) + (None,))
         err = np.abs(x.get(level) - ref).max() / np.abs(ref).max()
         assert err <= 1e-11, (captured, err)  # the bound of the sweeps' parity tests
 
