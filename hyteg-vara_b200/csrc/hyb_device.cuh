@@ -383,11 +383,14 @@ struct OpDev
 
 // How the constant operator's row reads its values: the loads of the valid offsets ahead of the
 // sums, those of all offsets (the position of an invalid one is some position of the slab),
-// or each load in its term's branch. FP32 surface rows read all: 27 us an interface colour at
-// level 6 on 384 cells against 33 for the valid ones; FP64 the valid ones: 20 us at level 7 on
-// 48 cells against 24, and an FP64 cycle on 6 cells, levels 0..5, whose row tables' passes
-// dominate: 497 us against 541. The apply, whose surface part is bound by the number of
-// gathers, keeps the branches: 271 us at level 6 on 384 cells against 281.
+// or each load in its term's branch. Surface rows of a sweep read all (sorIfaceBody,
+// k_surface_sor): a sweep with a launch per colour, valid ones against all, FP64 397 and 382 us
+// at level 7 on 48 cells, 596 and 534 at level 6 on 384, FP32 304 and 286, 390 and 359; with one
+// launch FP64 370 and 361, 487 and 482, FP32 278 and 268, 328 and 321. Row tables go by type
+// (rowLoads): an FP64 cycle on 6 cells, levels 0..5, 490 us with the valid ones against 526, on 384
+// cells 1449 against 1607; with FP32 cycles a solve on 6 cells 6.42 ms with all against 6.25, on 384
+// 20.7 against 20.5. The apply, whose surface part is bound by the number of gathers, keeps the
+// branches: 271 us at level 6 on 384 cells against 281 with the loads ahead.
 enum RowLoads : int
 {
    kRowValid  = 0,

@@ -934,7 +934,7 @@ __device__ __forceinline__ void sorIfaceBody( Blk vb, TopoDev tp, LevelDev lv, O
          own             = u[r0];
          b               = rhs[r0];
       }
-      bdryRowGroup< T, VAR >( tp, lv, op, u, p, tk, active, diag, off );
+      bdryRowGroup< T, VAR, kRowAll >( tp, lv, op, u, p, tk, active, diag, off );
       if ( !active )
          continue;
       const T v = ( T( 1 ) - relax ) * own + relax * ( b - off ) / diag;
@@ -942,8 +942,9 @@ __device__ __forceinline__ void sorIfaceBody( Blk vb, TopoDev tp, LevelDev lv, O
    }
 }
 
-// (constant operator, FP64 at level 7 on 48 cells: 26 us a colour with eight resident blocks, 20
-// with six and no spills; FP32 at level 6 on 384 cells: 27 with eight, 37 with six)
+// (constant operator. FP64, a whole sweep with six, seven and eight resident blocks, of which six do
+// not spill: level 7 on 48 cells 382, 386 and 405 us, level 6 on 36 cells 78, 79 and 83, on 384 cells
+// 534, 538 and 521. FP32 at level 6 on 384 cells: 27 us a colour with eight, 37 with six)
 template < typename T, int VAR >
 __global__ void __launch_bounds__( 128, VAR ? 4 : ( sizeof( T ) == 8 ? 6 : 8 ) ) k_sor_iface( TopoDev tp, LevelDev lv, OpDev< T > op, T* __restrict__ u,
                                                       const T* __restrict__ rhs, T relax, int flag, BdryLists bl )
