@@ -957,7 +957,7 @@ __global__ void __launch_bounds__( 128, VAR ? 4 : ( sizeof( T ) == 8 ? 6 : 8 ) )
 // residue block r = (c - 2y - 3z) mod 4, one contiguous run of the row; the colour's point
 // table lists them in storage order. Odd colours walk the cells in reverse order, so a
 // pass starts on the data the previous pass touched last (still in L2).
-template < typename T, int VAR >
+template < typename T, int VAR, bool KEEP = VAR == 1 >
 __device__ __forceinline__ void sorInteriorBody( Blk vb, TopoDev tp, LevelDev lv, OpDev< T > op, T* u,
                                                          const T* rhs, T relax, int colour, int begin,
                                                          int nPts, int nCellBlocks )
@@ -967,9 +967,11 @@ __device__ __forceinline__ void sorInteriorBody( Blk vb, TopoDev tp, LevelDev lv
    const int      nChunks = ( nPts + 32 * K - 1 ) / ( 32 * K );
    // strips only while every warp of the grid still gets at least one strip
    const int strip = max( 1, min( kInteriorStrip, tp.nC * nChunks / ( nCellBlocks * int( blockDim.x >> 5 ) ) ) );
-   // nodal coefficient: the cell's edge weights stay over the batches of a strip. The other
-   // operators load theirs for every batch: held across the loop they cost registers (FP64 154
-   // of them against 124, quadrature points 184 against 80) and resident blocks
+   // KEEP: the cell's weights stay over the batches of a strip. For the nodal coefficient, and in
+   // the constant operator's own kernel (FP64 at level 7 on 48 cells 355 us a sweep against 361); in
+   // the program kernels the constant weights would spill (a Jacobi cycle on 6 cells, levels 0..2, 76
+   // us against 73), and at quadrature points they cost registers alone (210 us a sweep at level 6 on
+   // 36 cells against 187)
    InteriorOp< T, VAR > io;
    int                  loaded = -1;
    HYB_CELL_LOOP_STRIP( nChunks, strip )
@@ -978,7 +980,7 @@ __device__ __forceinline__ void sorInteriorBody( Blk vb, TopoDev tp, LevelDev lv
       const int       cell = item / nChunks;
       PointBatch< K > pb;
       pb.load( pts, lv.blk, nPts, ( item - cell * nChunks ) * 32 * K + int( threadIdx.x & 31 ) );
-      if ( VAR != 1 || cell != loaded )
+      if ( !KEEP || cell != loaded )
          io.load( op, cell );
       loaded = cell;
       T*       uc = u + size_t( cell ) * lv.stride;
@@ -1006,15 +1008,18 @@ __device__ __forceinline__ void sorInteriorBody( Blk vb, TopoDev tp, LevelDev lv
    }
 }
 
-// (nodal coefficient: registers for four resident blocks in FP64 and six in FP32 without spills
-// to speak of; the others are left to the compiler, which takes up to 184 when asked for one block)
+// (nodal coefficient: registers for four resident blocks in FP64 and six in FP32 without spills to
+// speak of. The others: as many registers as the compiler likes, the loads of a row in flight count
+// for more than the blocks. A sweep with them and with its own choice of fewer, quadrature points
+// FP64 at level 6 on 384 cells 1725 and 1853 us, at level 5 on 48 cells 79 and 85 (at level 6 on 36
+// cells, however, 187 and 177); constant FP32 at level 5 on 48 cells 48 and 51, at level 7 282 and 268)
 template < typename T, int VAR >
-__global__ void __launch_bounds__( 128, VAR == 1 ? ( sizeof( T ) == 8 ? 4 : 6 ) : 0 ) k_sor_interior( TopoDev tp, LevelDev lv, OpDev< T > op, T* __restrict__ u,
+__global__ void __launch_bounds__( 128, VAR == 1 ? ( sizeof( T ) == 8 ? 4 : 6 ) : 1 ) k_sor_interior( TopoDev tp, LevelDev lv, OpDev< T > op, T* __restrict__ u,
                                                          const T* __restrict__ rhs, T relax, int colour, int begin,
                                                          int nPts, int nCellBlocks )
 {
    HYB_PDL_PROLOGUE();
-   sorInteriorBody< T, VAR >( launchBlk(), tp, lv, op, u, rhs, relax, colour, begin, nPts, nCellBlocks );
+   sorInteriorBody< T, VAR, VAR != 2 >( launchBlk(), tp, lv, op, u, rhs, relax, colour, begin, nPts, nCellBlocks );
 }
 
 // All four interior colour passes of a sweep in ONE launch for small levels: a block per
