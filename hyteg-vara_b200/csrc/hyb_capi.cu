@@ -1015,8 +1015,8 @@ int hyb_gmg_solve_to_tolerance( hyb_gmg* gh, hyb_function* xh, hyb_function* bh,
 namespace hyb {
 
 // 131072 partial sums = 1 MiB. Every GPU that loads this library holds the array until
-// the process exits. A call needs (closure size / 256, rounded up) x (#macro-cells)
-// slots; larger problems are rejected.
+// the process exits. Problems with more than that many slab values / 256 (rounded up per
+// macro-cell) are rejected; a call writes a quarter of it, one partial sum per 1024 values.
 constexpr int kNoAllocSlots = 131072;
 static __device__ __align__( 256 ) double g_noAllocPartial[kNoAllocSlots];
 

@@ -492,7 +492,8 @@ __device__ __forceinline__ void partialRow( const OpDev< T >& op, U u, int cell,
    const int         mask  = classMask( N, x, y, z );
    const uint32_t    valid = kValidOffsets[mask];
    const StencilRows R     = stencilRows( W, y, z );
-   // positions of the neighbours inside the closure (the others are never read)
+   // positions of the neighbours inside the closure; the others are 0, where a row that reads all
+   // offsets reads a value it drops
    int pos[15];
 #pragma unroll
    for ( int q = 0; q < 15; ++q )

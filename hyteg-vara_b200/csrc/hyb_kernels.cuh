@@ -2155,7 +2155,7 @@ __global__ void __launch_bounds__( 128 ) k_restrict( TopoDev tp, LevelDev lv, in
 // Pointwise vector kernels over whole cell slabs (all replicas; consistent by
 // construction). blockIdx.y = cell. They are DRAM bound once a thread has several 16-byte
 // loads in flight and the per-point work is small: a thread takes kVecWidth consecutive
-// values (slabs start on 256-byte boundaries), and the boundary flags of the cell's 16
+// values (slabs start on 128-byte boundaries), and the boundary flags of the cell's 16
 // point classes are read once per block into a 16-bit mask instead of once per point. One
 // value per thread with a class-table read per point took 125 us for a two-term FP64
 // combination of 18.4 M slab values (3.5 TB/s) and 103 us for a dot product (2.9 TB/s), and

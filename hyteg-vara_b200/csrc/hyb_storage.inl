@@ -114,7 +114,10 @@ inline int stridePad( int s ) { return ( s + 31 ) / 32 * 32; }
 // The interface colours of a level run as one cooperative launch (hyb_surface.cu) from this many
 // surface DoFs on (HYB_SURFACE_MIN_DOFS overrides it). At level 6 on 48 cells (0.25 M) a sweep's
 // six launches take 40 us and the one 61; at level 7 on 48 cells (1 M) 130 against 100, at level
-// 6 on 384 cells (1.8 M, FP32) 165 against 130.
+// 6 on 384 cells (1.8 M, FP32) 165 against 130. Upwards it ends where a block's faces no longer fit
+// its shared memory: with 148 SMs at 740 inner faces at level 6 and 148 at level 7 in FP64 (about
+// 430 and 96 cells of a cuboid), at twice as many in FP32. Beyond that, and on levels above 7, a
+// colour has its launch.
 constexpr long kSurfaceMinDofs = 500000;
 inline long    surfaceMinDofs()
 {

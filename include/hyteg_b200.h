@@ -165,8 +165,8 @@ int hyb_function_copy_convert( hyb_function* dst, hyb_function* src, int level, 
  * while they run (a serving loop bound to a fixed HBM budget, a host framework that owns
  * the allocator). No counterpart in the reference. It allocates nothing: its scratch is
  * a 1 MiB file-scope device array that every GPU loading this library holds until exit,
- * so problems needing more than 131072 partial sums ((closure size / 256, rounded up) x
- * #macro-cells) are rejected with HYB_EINVAL. Asynchronous on `stream`; the result is
+ * so problems with (closure size / 256, rounded up) x #macro-cells above 131072 are
+ * rejected with HYB_EINVAL. Asynchronous on `stream`; the result is
  * written to the device double `out_device`. The first call on a device looks up the
  * array's device address with that device current; make that first call before any
  * stream capture. All calls share the array and it keeps the last call's contents:
