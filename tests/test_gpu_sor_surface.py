@@ -5,7 +5,7 @@ The launch takes over at half a million surface DoFs; here HYB_SURFACE_MIN_DOFS 
 a child process, so that it runs on: the smallest levels it takes (faces of 21 points), six
 macro-tets (every face cut into row ranges, fewer blocks than SMs), the 48-tet cuboid (as many
 ranges as SMs), a 144-tet box (several whole faces per block), level 7 and the spherical shell
-(ten colours). Whole sweeps, forward and backward, relax 1 and 0.8. The rows are summed in
+(seven colours). Whole sweeps, forward and backward, relax 1 and 0.8. The rows are summed in
 another order than the oracle's, in the sweep's precision: 1e-11 in FP64 (max norm, relative),
 the bound of the sweeps' parity tests; 2e-5 for two FP32 sweeps."""
 import os
@@ -57,6 +57,31 @@ def test_interface_passes_match_oracle(mesh, level):
                PYTHONPATH=os.pathsep.join([os.path.join(ROOT, "oracle"), os.path.join(ROOT, "hyteg-vara_b200", "python")]))
     r = subprocess.run([sys.executable, os.path.abspath(__file__), mesh, str(level)], env=env, capture_output=True, text=True)
     assert r.returncode == 0, r.stderr[-2000:]
+
+
+@pytest.mark.gpu
+def test_large_meshes_leave_the_one_launch_by_type():
+    """848 inner faces at level 6 are six a block: 114 KB in FP32, which runs in one launch, and
+    206 KB, more than the limit, in FP64, which takes a launch per colour. The two agree to the bound of
+    the FP32 sweep above."""
+    import hyteg_b200 as H
+
+    level = 6
+    st = H.PrimitiveStorage.cuboid(4, 4, 5, level)
+    A = H.P1ConstantLaplaceOperator(st, level, level)
+    m, _ = st.colouring()
+    rng = np.random.default_rng(1)
+    x0, b = (rng.uniform(-1, 1, st.num_dofs(level)).astype(np.float32) for _ in range(2))
+    got = []
+    for dtype, launches in ((H.F64, m + 4), (H.F32, 1 + 4)):
+        fx, fb = H.P1Function("x", st, level, level, dtype), H.P1Function("b", st, level, level, dtype)
+        fx.set(x0, level)
+        fb.set(b, level)
+        n = H.load().hyb_kernel_launch_count()
+        A.smooth_sor(fx, fb, 0.8, level, H.INNER | H.NEUMANN)
+        assert H.load().hyb_kernel_launch_count() - n == launches
+        got.append(fx.get(level).astype(np.float64))
+    assert np.abs(got[1] - got[0]).max() <= 2e-5 * np.abs(got[0]).max()
 
 
 if __name__ == "__main__":
