@@ -177,10 +177,7 @@ void buildSurface( const Storage& s, LevelHost& lh )
       sf.most  = std::max( sf.most, ( held + 7 ) / 8 * 8 );
       sf.tiles = std::max( sf.tiles, off[size_t( b ) + 1] - off[size_t( b )] );
    }
-   bool fits = sf.tiles <= kSurfaceMaxTiles && surfaceSmem( sf, sizeof( float ) ) <= kSurfaceMaxSmem;
-   if ( fits )
-      HYB_CUDA( surfacePrepare( sf, &fits ) );
-   if ( !fits )
+   if ( sf.tiles > kSurfaceMaxTiles || surfaceSmem( sf, sizeof( float ) ) > kSurfaceMaxSmem || !surfacePrepare( sf ) )
    {
       sf = SurfaceDev{};
       return;

@@ -378,20 +378,20 @@ __global__ void __launch_bounds__( kSurfaceThreads, 1 )
 size_t surfaceSmem( const SurfaceDev& sf, int elem ) { return size_t( sf.most ) * ( 2 * elem + 2 ) + 16; }
 
 namespace {
-// one block of every SM of the current device has room for the launch in T, and the opt-in to its
-// shared memory is set
+// the opt-in to the launch's shared memory in T is set, and the SMs of the current device have room
+// for its blocks (a value type whose tiles do not fit is refused by surfaceSor)
 template < typename T >
-cudaError_t prepareFor( const SurfaceDev& sf, int sms, bool* fits )
+bool prepareFor( const SurfaceDev& sf, int sms )
 {
-   const cudaError_t e =
-       cudaFuncSetAttribute( k_surface_sor< T >, cudaFuncAttributeMaxDynamicSharedMemorySize, int( kSurfaceMaxSmem ) );
-   if ( e != cudaSuccess || surfaceSmem( sf, sizeof( T ) ) > kSurfaceMaxSmem )
-      return e; // (the value types are asked for one by one: surfaceSor)
-   int               perSM = 0;
-   const cudaError_t o     = cudaOccupancyMaxActiveBlocksPerMultiprocessor( &perSM, k_surface_sor< T >, kSurfaceThreads,
-                                                                        surfaceSmem( sf, sizeof( T ) ) );
-   *fits                   = *fits && perSM * sms >= sf.nBlocks;
-   return o;
+   if ( cudaFuncSetAttribute( k_surface_sor< T >, cudaFuncAttributeMaxDynamicSharedMemorySize, int( kSurfaceMaxSmem ) ) !=
+        cudaSuccess )
+      return false;
+   if ( surfaceSmem( sf, sizeof( T ) ) > kSurfaceMaxSmem )
+      return true;
+   int perSM = 0;
+   return cudaOccupancyMaxActiveBlocksPerMultiprocessor( &perSM, k_surface_sor< T >, kSurfaceThreads,
+                                                         surfaceSmem( sf, sizeof( T ) ) ) == cudaSuccess &&
+          perSM * sms >= sf.nBlocks;
 }
 
 // SMs of the context (or its partition) that the stream's kernels run on; 0 where the driver
@@ -431,22 +431,17 @@ int streamSMs( cudaStream_t stream )
 }
 } // namespace
 
-cudaError_t surfacePrepare( const SurfaceDev& sf, bool* fits )
+bool surfacePrepare( const SurfaceDev& sf )
 {
-   int         dev = 0, coop = 0, mps = 0, sms = 0;
-   cudaError_t e   = cudaGetDevice( &dev );
-   if ( e == cudaSuccess )
-      e = cudaDeviceGetAttribute( &coop, cudaDevAttrCooperativeLaunch, dev );
-   if ( e == cudaSuccess )
-      e = cudaDeviceGetAttribute( &mps, cudaDevAttrMpsEnabled, dev );
-   if ( e == cudaSuccess )
-      e = cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev );
-   *fits = coop && !mps;
-   if ( e == cudaSuccess )
-      e = prepareFor< float >( sf, sms, fits );
-   if ( e == cudaSuccess )
-      e = prepareFor< double >( sf, sms, fits );
-   return e;
+   int        dev = 0, coop = 0, mps = 0, sms = 0;
+   const bool ok  = cudaGetDevice( &dev ) == cudaSuccess &&
+                   cudaDeviceGetAttribute( &coop, cudaDevAttrCooperativeLaunch, dev ) == cudaSuccess && coop &&
+                   cudaDeviceGetAttribute( &mps, cudaDevAttrMpsEnabled, dev ) == cudaSuccess && !mps &&
+                   cudaDeviceGetAttribute( &sms, cudaDevAttrMultiProcessorCount, dev ) == cudaSuccess &&
+                   prepareFor< float >( sf, sms ) && prepareFor< double >( sf, sms );
+   if ( !ok )
+      cudaGetLastError(); // a query the device or driver refuses is an answer, not an error of the storage
+   return ok;
 }
 
 template < typename T >

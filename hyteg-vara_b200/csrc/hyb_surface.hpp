@@ -38,7 +38,7 @@ constexpr size_t kSurfaceMaxSmem = 200 * 1024;
 // every storage that has tiles calls this when it is built) and tells whether the device can run
 // it: with room for the whole grid, and not under MPS, where a cooperative launch is not allowed
 // in the body of a graph's loop, as the device-iterated solves have it.
-cudaError_t surfacePrepare( const SurfaceDev& sf, bool* fits );
+bool surfacePrepare( const SurfaceDev& sf );
 
 // All interface colours of one sweep (in the order 0 .. m-1, backwards: m-1 .. 0), for the
 // DoFs on Inner | Neumann. A cooperative launch; cudaErrorCooperativeLaunchTooLarge, captured or

@@ -61,6 +61,8 @@ cudaError_t cudaGetDevice( int* d )
 cudaError_t cudaGetLastError() { return cudaSuccess; }
 cudaError_t cudaDeviceGetAttribute( int* v, cudaDeviceAttr a, int )
 {
+   if ( fake.refuses )
+      return cudaErrorInvalidValue;
    *v = a == cudaDevAttrCooperativeLaunch ? fake.cooperative : a == cudaDevAttrMpsEnabled ? fake.mps : fake.sms;
    return cudaSuccess;
 }

@@ -11,6 +11,7 @@ struct FakeCuda
    int perSM       = 1;   // resident blocks of any kernel per SM
    int ctxSMs      = 148; // of a stream's context
    int greenSMs    = 0;   // of a stream's green context (0: it has none)
+   bool refuses    = false; // attribute queries fail
    bool noDriver   = false; // the driver's entry points are not found
 };
 extern FakeCuda fake;

@@ -39,8 +39,7 @@ int devices()
    const SurfaceDev sf = tiles();
    for ( fake.device = 0; fake.device < 2; ++fake.device )
    {
-      bool fits = false;
-      CHECK( surfacePrepare( sf, &fits ) == cudaSuccess && fits );
+      CHECK( surfacePrepare( sf ) );
       CHECK( launch< double >( sf ) == cudaSuccess );
       CHECK( launch< float >( sf ) == cudaSuccess );
    }
@@ -55,13 +54,13 @@ int fits()
    auto kept = []( auto&& change ) {
       fake = FakeCuda{};
       change();
-      bool f = false;
-      return surfacePrepare( tiles(), &f ) == cudaSuccess && f;
+      return surfacePrepare( tiles() );
    };
    CHECK( kept( [] {} ) );
    CHECK( !kept( [] { fake.mps = 1; } ) );
    CHECK( !kept( [] { fake.cooperative = 0; } ) );
    CHECK( !kept( [] { fake.perSM = 0; } ) );
+   CHECK( !kept( [] { fake.refuses = true; } ) ); // and the storage is built all the same
    CHECK( !kept( [] { fake.sms = 147; } ) );
    CHECK( kept( [] { fake.sms = 74, fake.perSM = 2; } ) );
    return 0;
@@ -72,10 +71,9 @@ int stream()
 {
    const SurfaceDev sf = tiles();
    auto             launched = [&]( auto&& change ) {
-      fake     = FakeCuda{};
-      bool   f = false;
+      fake = FakeCuda{};
       change();
-      return surfacePrepare( sf, &f ) == cudaSuccess && launch< float >( sf ) == cudaSuccess && fake.launches == 1;
+      return surfacePrepare( sf ) && launch< float >( sf ) == cudaSuccess && fake.launches == 1;
    };
    CHECK( launched( [] {} ) );
    CHECK( !launched( [] { fake.greenSMs = 64; } ) );
@@ -89,8 +87,7 @@ int stream()
 int silent()
 {
    fake.noDriver = true;
-   bool f        = false;
-   CHECK( surfacePrepare( tiles(), &f ) == cudaSuccess );
+   CHECK( surfacePrepare( tiles() ) );
    CHECK( launch< double >( tiles() ) == cudaErrorCooperativeLaunchTooLarge && fake.launches == 0 );
    return 0;
 }
