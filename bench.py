@@ -288,7 +288,7 @@ def ours(args, rank, world, local_rank):
                 "peak_source": peak_kind, "traffic": t_bytes, "traffic_source": t_src}
 
     # DRAM bytes (read + write) per launch from the warm-cache ncu captures of the same kernels
-    # and workload that profiles/ summarises (one sweep = the sum over its ten launches)
+    # and workload that profiles/ summarises (one sweep = the sum over its five launches)
     sweep_prof, apply_prof = "k_sor_fp64_fp32_level7_cube48.md", "k_apply_fp64_level7_cube48.md"
     sweep64_traffic = profile_figure(sweep_prof, "fp64_sweep_bytes")
     sweep32_traffic = profile_figure(sweep_prof, "fp32_sweep_bytes")
@@ -374,12 +374,12 @@ def ours(args, rank, world, local_rank):
             "error_mixed_vs_fp64_solution": err_mixed,
             "dof_updates_per_s_fp64": world * n_unknowns * sum(cyc_fp64) / (t_fp64 / 1e3),
             "roofline": dict(roof(sor_gbs, sweep64_traffic, "ncu (warm caches), profiles/" + sweep_prof),
-                             kernel="k_sor_iface + k_sor_interior (one FP64 multicolour SOR sweep, 10 launches, level 7)",
+                             kernel="k_surface_sor + k_sor_interior (one FP64 multicolour SOR sweep, 5 launches, level 7)",
                              ms=t_sor * 1e3),
             "roofline_apply": dict(roof(apply_gbs, apply_traffic, "ncu (warm caches), profiles/" + apply_prof),
                                    kernel="k_apply (FP64 stencil apply, level 7)", ms=t_apply * 1e3),
             "roofline_sor_fp32": dict(roof(sor32_gbs, sweep32_traffic, "ncu (warm caches), profiles/" + sweep_prof),
-                                      kernel="k_sor_iface + k_sor_interior (FP32 sweep, level 7)", ms=t_sor32 * 1e3),
+                                      kernel="k_surface_sor + k_sor_interior (FP32 sweep, level 7)", ms=t_sor32 * 1e3),
             "reference_order_fp64": ref_order,
             "e2e": e2e, "gpu_launches": launches, "clocks": clocks, "cpu_baseline": cpu,
             "variable_coefficient": varcoef, "spherical_shell": shell, "blended_shell": blend, "serving": serve,
