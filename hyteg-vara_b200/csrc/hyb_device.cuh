@@ -391,6 +391,8 @@ struct OpDev
 // cells 1449 against 1607; with FP32 cycles a solve on 6 cells 6.42 ms with all against 6.25, on 384
 // 20.7 against 20.5. The apply, whose surface part is bound by the number of gathers, keeps the
 // branches: 271 us at level 6 on 384 cells against 281 with the loads ahead.
+// At quadrature points the choice is between the factors of all micro-tets (kRowAll) and of the
+// valid ones (rowVariable).
 enum RowLoads : int
 {
    kRowValid  = 0,
@@ -435,10 +437,13 @@ __device__ __forceinline__ void rowConstant( const T* st, uint32_t valid, T& dia
 // variable coefficient: the offsets `valid` and micro-tets validT around the point; at(q) is the
 // slab position of offset q. The weights of the 14 edges are collected over the tets (three per tet), the
 // off-diagonal sum takes one product per edge, and the diagonal is minus the sum of the
-// weights (the element matrices have zero row sums and are symmetric: one entry per pair). Only
-// the factors of the valid micro-tets are read at quadrature points (half of the 24 on a face): an
-// FP32 residual at level 6 on 384 cells takes 639 us, with all 24 read 836.
-template < typename T, int VAR, typename Val, typename At >
+// weights (the element matrices have zero row sums and are symmetric: one entry per pair). At
+// quadrature points ALL reads the factors of all 24 micro-tets, else those of the valid ones (half
+// of them on a face): FP32 residual at level 6 on 384 cells 836 us with all, 639 with the valid
+// ones, an FP64 cycle on 6 cells, levels 0..5, 1094 against 686. The reference-order sweep, a chain of
+// single rows, reads all (FP32 at level 5 on 6 cells 242 us against 315), and so do the FP64 Jacobi
+// rows (a cycle on 6 cells, levels 0..5, 297 against 307).
+template < typename T, int VAR, bool ALL, typename Val, typename At >
 __device__ __forceinline__ void rowVariable( const OpDev< T >& op, int cell, uint32_t valid, uint32_t validT, T& diag,
                                              T& off, Val&& val, At&& at )
 {
@@ -462,9 +467,10 @@ __device__ __forceinline__ void rowVariable( const OpDev< T >& op, int cell, uin
       const bool        in = validT & ( 1u << i );
       T                 ks;
       if constexpr ( VAR == 2 )
-         ks = in ? op.kq[( size_t( cell ) * 6 + it.t ) * op.stride + at( it.q[0] )] : T( 0 );
+         ks = ALL || in ? op.kq[( size_t( cell ) * 6 + it.t ) * op.stride + at( it.q[0] )] : T( 0 );
       else
-         ks = in ? kq[it.q[0]] + kq[it.q[1]] + kq[it.q[2]] + kq[it.q[3]] : T( 0 );
+         ks = kq[it.q[0]] + kq[it.q[1]] + kq[it.q[2]] + kq[it.q[3]];
+      ks = in ? ks : T( 0 );
 #pragma unroll
       for ( int j = 0; j < 4; ++j )
          if ( j != it.k )
@@ -507,7 +513,7 @@ __device__ __forceinline__ void partialRow( const OpDev< T >& op, U u, int cell,
       rowConstant< T, LOADS >( st, valid, diag, off, [&]( int q ) { return u[pos[q]]; } );
    }
    else
-      rowVariable< T, VAR >( op, cell, valid, kValidTets[mask], diag, off, [&]( int q ) { return u[pos[q]]; }, [&]( int q ) { return pos[q]; } );
+      rowVariable< T, VAR, LOADS == kRowAll >( op, cell, valid, kValidTets[mask], diag, off, [&]( int q ) { return u[pos[q]]; }, [&]( int q ) { return pos[q]; } );
 }
 
 } // namespace hyb

@@ -634,7 +634,7 @@ __device__ __forceinline__ void rowPassBody( const RowPass& rp, const OpDev< T >
          {
             // base = cell * stride
             const int cls = ( A.y / 15 ) & 15, cell = A.y / 240;
-            rowVariable< T, VAR >( op, cell, valid, kValidTets[cls], diag, off, [&]( int q ) { return uc[pos( q )]; }, pos );
+            rowVariable< T, VAR, MODE == kRowJacobi && sizeof( T ) == 8 >( op, cell, valid, kValidTets[cls], diag, off, [&]( int q ) { return uc[pos( q )]; }, pos );
          }
       }
       const int G = gt < rp.b1 ? 32 : gt < rp.b2 ? 8 : gt < rp.b3 ? 2 : 1;
@@ -934,7 +934,7 @@ __device__ __forceinline__ void sorIfaceBody( Blk vb, TopoDev tp, LevelDev lv, O
          own             = u[r0];
          b               = rhs[r0];
       }
-      bdryRowGroup< T, VAR, kRowAll >( tp, lv, op, u, p, tk, active, diag, off );
+      bdryRowGroup< T, VAR, VAR == 2 ? kRowValid : kRowAll >( tp, lv, op, u, p, tk, active, diag, off );
       if ( !active )
          continue;
       const T v = ( T( 1 ) - relax ) * own + relax * ( b - off ) / diag;
@@ -1151,7 +1151,7 @@ __global__ void __launch_bounds__( 128 ) k_sorref_vertices( TopoDev tp, LevelDev
       const BdryPoint p      = decodeBdry( tp, lv, tk.t );
       const bool      active = tk.valid && ( primBc( tp, p.kind, p.prim ) & flag );
       T               diag, off;
-      bdryRowGroup< T, VAR >( tp, lv, op, snap, p, tk, active, diag, off );
+      bdryRowGroup< T, VAR, VAR == 2 ? kRowAll : rowLoads< T >() >( tp, lv, op, snap, p, tk, active, diag, off );
       if ( !active )
          continue;
       const size_t r0 = bdryReplica< T >( tp, lv, p, 0 );
@@ -1296,7 +1296,7 @@ __global__ void __launch_bounds__( sorRefCellThreads( VAR ) ) k_sorref_cells( To
          const int     i   = sidx( lv.W, x, y, z );
          const T       own = uc[i], bb = bc[i];
          T             diag = 0, off = 0;
-         partialRow< T, VAR >( op, uc, c, lv.W, x, y, z, diag, off );
+         partialRow< T, VAR, VAR == 2 ? kRowAll : rowLoads< T >() >( op, uc, c, lv.W, x, y, z, diag, off );
          uc[i] = ( T( 1 ) - relax ) * own + relax * ( bb - off ) / diag;
       }
       __syncthreads();
