@@ -843,20 +843,32 @@ __device__ __forceinline__ void applyBody( Blk vb, TopoDev tp, LevelDev lv, OpDe
       const LaneTask  tk     = laneTask( tp, lv, bl, gt );
       const BdryPoint p      = decodeBdry( tp, lv, tk.t );
       const bool      active = tk.valid && ( primBc( tp, p.kind, p.prim ) & flag );
-      T               diag, off, v = 0;
-      bdryRowGroup< T, VAR, kRowBranch >( tp, lv, op, src, p, tk, active, diag, off );
-      // The point's own value is read after the sums, as held through them it spills: FP64 at level 7
-      // on 48 cells 199 us an apply against 195, a residual 218 against 214.
-      if ( active )
+      // The point's own value and dst's or rhs's travel with the row's loads, but for the constant
+      // operator in FP64, which spills when it holds them through the sums: at level 7 on 48 cells
+      // 199 us an apply with them first against 195, a residual 218 against 214, an additive apply 244
+      // against 241 (6 cells at level 5: 6.0 against 6.3), and for the plain apply, which gains
+      // nothing. FP32 at level 5 on 48 cells: additive apply 9.7 us with them first, 10.4 after the
+      // sums; nodal coefficient, level 6 on 384 cells, FP64: residual 840 against 861.
+      constexpr bool early = MODE != kReplace && !( sizeof( T ) == 8 && VAR == 0 );
+      T              diag, off, v = 0, own = 0, b = 0;
+      if ( early && active )
       {
          const size_t r0 = bdryReplica< T >( tp, lv, p, 0 );
-         const T      ax = diag * src[r0] + off;
-         if constexpr ( MODE == kReplace )
-            v = ax;
-         else if constexpr ( MODE == kAdd )
-            v = dst[r0] + ax;
-         else
-            v = rhs[r0] - ax;
+         own             = src[r0];
+         b               = MODE == kAdd ? dst[r0] : rhs[r0];
+      }
+      bdryRowGroup< T, VAR, kRowBranch >( tp, lv, op, src, p, tk, active, diag, off );
+      if ( active )
+      {
+         if ( !early )
+         {
+            const size_t r0 = bdryReplica< T >( tp, lv, p, 0 );
+            own             = src[r0];
+            if constexpr ( MODE != kReplace )
+               b = MODE == kAdd ? dst[r0] : rhs[r0];
+         }
+         const T ax = diag * own + off;
+         v          = MODE == kReplace ? ax : MODE == kAdd ? b + ax : b - ax;
       }
       __syncwarp(); // every lane of a group has read dst[r0] or rhs[r0] before a replica is written
       if ( !active )
