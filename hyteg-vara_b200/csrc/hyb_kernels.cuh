@@ -1969,9 +1969,10 @@ __device__ __forceinline__ void jacobiBody( Blk vb, TopoDev tp, LevelDev lv, OpD
       const BdryPoint p      = decodeBdry( tp, lv, tk.t );
       const bool      active = tk.valid && ( primBc( tp, p.kind, p.prim ) & flag );
       T               diag, off;
-      // constant operator, 6 to 384 cells: FP64 with the branches 35.0 us at level 6 on 36 cells, loads
-      // ahead 35.6; FP32 with all loads ahead 25.3, with the branches 27.2
-      bdryRowGroup< T, VAR, sizeof( T ) == 8 ? kRowBranch : kRowAll >( tp, lv, op, src, p, tk, active, diag, off );
+      // constant operator, with all loads ahead and with a branch per term: level 6 on 384 cells FP64
+      // 370 and 404 us, FP32 270 and 300, 6 cells at level 3 FP64 4.4 and 5.3. At quadrature points all
+      // factors in FP64, the valid ones in FP32 (level 6 on 36 cells 63.5 and 59.8 us)
+      bdryRowGroup< T, VAR, VAR == 2 && sizeof( T ) == 4 ? kRowValid : kRowAll >( tp, lv, op, src, p, tk, active, diag, off );
       if ( !active )
          continue;
       const size_t r0 = bdryReplica< T >( tp, lv, p, 0 );
@@ -1980,10 +1981,8 @@ __device__ __forceinline__ void jacobiBody( Blk vb, TopoDev tp, LevelDev lv, OpD
    }
 }
 
-// (variable coefficient, FP64: four resident blocks; left alone the registers of its surface rows
-// leave three. Level 6 on 384 cells: nodal 746 us against 887, quadrature points 917 against 1100)
 template < typename T, int VAR >
-__global__ void __launch_bounds__( 128, VAR && sizeof( T ) == 8 ? 4 : 0 ) k_jacobi( TopoDev tp, LevelDev lv, OpDev< T > op, const T* __restrict__ src,
+__global__ void __launch_bounds__( 128 ) k_jacobi( TopoDev tp, LevelDev lv, OpDev< T > op, const T* __restrict__ src,
                                                    T* __restrict__ dst, const T* __restrict__ rhs, T relax, int flag,
                                                    int nCellBlocks )
 {
