@@ -2573,8 +2573,10 @@ __global__ void k_reduce_final( const double* __restrict__ partial, int n, doubl
 // interior, the blocks behind them, over all cells, the surface DoFs, a thread each. Deriving
 // every point's canonical number from its coordinates (class table, tetrahedral indices) was
 // issue bound: 98 us for 18.4 M slab values in FP64 and 93 us in FP32, now 45 and 34 us.
+// (FP32: registers for eight resident blocks, an upload at level 6 on 384 cells 39.8 us against 45;
+// FP64 is left alone: 77 us, with eight 83)
 template < typename T, bool TO >
-__global__ void __launch_bounds__( kVecThreads ) k_dofs( TopoDev tp, LevelDev lv, int nIntBlocks, T* __restrict__ slab,
+__global__ void __launch_bounds__( kVecThreads, sizeof( T ) == 4 ? 8 : 0 ) k_dofs( TopoDev tp, LevelDev lv, int nIntBlocks, T* __restrict__ slab,
                                                          T* __restrict__ dofs )
 {
    HYB_PDL_PROLOGUE();
